@@ -106,6 +106,38 @@ __host__ __device__ inline bool conv_staging(int ci, int h, int wd, int kh, int 
   return true;
 }
 
+// Whole-plane staging (3 x 3 windows on images whose rows the TMA cannot describe: 14 x 14 and 7 x 7 at any
+// batch).  The planes of `cc` consecutive channels of one image are contiguous in memory, so one untiled bulk
+// copy per image brings a slot's channels -- no tensor map, no alignment rule on the rows; a channel count that
+// is a multiple of 4 keeps every copy on 16 bytes.  A tile is 128 consecutive output pixels of the whole batch,
+// which may lie in up to `imgs` images; there is no zero fill, so taps outside the image are masked when they
+// are read.  Fills `st` (slot_bytes: one image's part of a slot) and returns how many images a slot holds, 0 if
+// the conv does not qualify.
+__host__ __device__ inline int conv_plane_staging(int n, int ci, int h, int wd, int kh, int kw, int stride, int pad, int oh, int ow, ConvStaging *st) {
+  // (slots start 2 KB into the window and 16 KB of weights follow the last one: a tap up to two rows outside
+  // its plane stays inside the window)
+  if (kh != 3 || kw != 3 || ci % 32 || pad > 2 || wd > 64) return 0;
+  const int ohw = oh * ow;
+  // 128 consecutive pixels of the batch touch up to `span` images; where their planes would leave the raw ring
+  // fewer than six slots, tiles of whole images (49-pixel outputs of a 14 x 14 input: two instead of four)
+  const int span = (ohw - 1 + kConvBN - 1) / ohw + 1, whole = kConvBN / ohw;
+  st->tile_px = kConvBN;
+  int imgs = span < n ? span : n;
+  if (whole > 0 && whole < imgs && imgs * h * wd * 16 > 8 * 1024) st->tile_px = whole * ohw, imgs = whole;
+  int cc = 4;
+  if (imgs * cc * h * wd * 4 > 16 * 1024) return 0;
+  while (cc < 32 && imgs * 2 * cc * h * wd * 4 <= 8 * 1024) cc *= 2;
+  st->slots = 3;
+  st->cc = cc;
+  st->rows = h, st->pitch = wd;
+  st->ex = st->ey = 1;
+  st->step_x = st->step_y = stride;
+  st->x_start = 0, st->x_off = -pad;
+  st->slot_bytes = cc * h * wd * 4;
+  st->slot_pitch = (imgs * st->slot_bytes + 127) / 128 * 128;
+  return imgs;
+}
+
 struct ConvUmmaParams {
   alignas(64) CUtensorMap map_w;    // {K, co, 1}, box {32 fp32, 128, 1}, 128B swizzle
   alignas(64) CUtensorMap map_out;  // {oh*ow, co, n}, box {32 fp32, 32, 1}, 128B swizzle (stores); unused when oh*ow % 4 != 0
@@ -120,6 +152,7 @@ struct ConvUmmaParams {
   int kb_per_slice;     // K blocks per k-slice
   int ctas;             // staged: CTAs of the grid (a CTA takes every ctas-th tile)
   ConvStaging st;       // st.slots == 0: gathered from global memory
+  int plane_imgs;       // > 0: staged as whole planes of up to this many images per slot (conv_plane_staging)
   long long *timeline;  // diagnostic: when non-null, CTA 0 records globaltimer marks (UmmaMark indices)
 };
 
@@ -146,9 +179,21 @@ __host__ __device__ inline bool conv_staged_ring(int smem, int K, int kslot, int
   *slots = s, *wstages = w;
   return w >= (num_kb < 2 ? num_kb : 2);
 }
-__host__ __device__ inline int conv_staged_smem_bytes(int K, int slots, int slot_pitch, int wstages) {
-  return conv_header_bytes(K) + conv_raw_bytes(slots, slot_pitch) + wstages * kUmmaABytes;
+__host__ __device__ inline int conv_staged_smem_bytes(int header, int slots, int slot_pitch, int wstages) {
+  return header + conv_raw_bytes(slots, slot_pitch) + wstages * kUmmaABytes;
 }
+// The whole-plane form with the K range split over a cluster: once the MMAs are done the two rings receive the
+// partial sums of the 16-channel groups a CTA owns, 8 / split groups from each of split CTAs.
+// Raw slots of the whole-plane form in a window of `smem` bytes: what the header and the four weight stages
+// leave, up to 6, never more than a tile loads; 0: the window is too small.
+__host__ __device__ inline int conv_plane_slots(int smem, int Kslice, int cc, int slot_pitch) {
+  const int room = smem - kUmmaHeaderBytes - kConvAStages * kUmmaABytes, loads = Kslice / (9 * cc);
+  int s = loads < kConvMaxRawSlots ? loads : kConvMaxRawSlots;
+  while (s > 0 && conv_raw_bytes(s, slot_pitch) > room) --s;
+  return s >= (loads < 2 ? loads : 2) ? s : 0;
+}
+constexpr int kConvGroupBytes = 16 * kUmmaBM * 4;   // one CTA's fp32 partial of 16 channels x 128 pixels
+__host__ __device__ constexpr int conv_plane_recv_bytes(int split) { return split > 1 ? 8 * kConvGroupBytes : 0; }
 
 // 4-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros instead
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const float *src, uint32_t src_bytes) {
@@ -166,6 +211,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
+}
+// untiled bulk copy global -> shared; both addresses and the size are multiples of 16 bytes
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 // has phase `parity` of the barrier completed?  Never blocks.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
@@ -270,31 +320,29 @@ struct ConvUmmaTf32 {
   // where the four-channel walk stands, across the tiles of a CTA
   struct SlotWalk {
     uint32_t rs = 0, rph = 0;   // raw slot of the next step, its phase
-    int quad_in_slot = 0;       // a slot of more than 4 channels is walked in `quads` steps of 4
     int kdone = 0;              // values of k written so far (over all tiles: the A ring's column is kdone mod 128)
-    int acquired = 0;           // A stages (counted over all tiles) whose "empty" has been seen
   };
-  template <bool PAIR>
-  __device__ __forceinline__ static bool repack_3x3(const TileCtx &c, int K, bool lane0, const unsigned char *rawpix_p, uint32_t slot_pitch,
-                                                    int nslots, int quads, uint32_t plane4, uint32_t pitch4, uint32_t a_row, uint32_t raw_full0,
-                                                    uint32_t raw_empty0, uint32_t a_full0, uint32_t a_empty0, SlotWalk &walk) {
+  // Both barriers a step needs are asked ahead: the next raw slot while this step's reads travel, the A stage before
+  // the reads, which the answer would otherwise queue behind (commits arrive in order, so the last stage's stands
+  // for all).  Steps of eight channels pay those costs half as often and were no faster: two of them do not fit the
+  // 128-column A ring, so every step waits for the MMAs of the one before.
+  // MASK (whole planes, which have no zero fill around them): taps[3 dy + dx] is all ones where the tap lies inside
+  // the image, else 0.
+  template <bool PAIR, bool MASK>
+  __device__ __forceinline__ static bool repack_3x3(const TileCtx &c, int K, const unsigned char *rawpix_p, uint32_t slot_pitch,
+                                                       int nslots, int quads, uint32_t plane4, uint32_t pitch4, uint32_t a_row,
+                                                       uint32_t raw_full0, uint32_t raw_empty0, uint32_t full0, uint32_t empty0, SlotWalk &walk,
+                                                       const uint32_t (&taps)[9]) {
     int *const status = c.status;
-    const int steps = K / 36;
+    const int steps = K / 36, lane = threadIdx.x & 31;
     uint32_t rs = walk.rs, rph = walk.rph;
-    int quad_in_slot = walk.quad_in_slot, kdone = walk.kdone, acquired = walk.acquired;
-    bool seen_raw = false, seen_empty = false;
+    int quad_in_slot = 0, kdone = walk.kdone;   // a slot of more than 4 channels is walked in `quads` steps of 4
+    bool raw_seen = false;   // this step's slot has been seen full
     for (int s = 0; s < steps; ++s) {
-      if (quad_in_slot == 0 && !seen_raw && !warp_wait(lane0, raw_full0 + 8 * rs, rph, status, UMMA_WAIT_FULL_TIMEOUT)) return false;
-      // the stages this slot's 36 columns fall into: kdone / 32 and, mostly, the one after
+      if (!raw_seen && quad_in_slot == 0 && !warp_wait(lane == 0, raw_full0 + 8 * rs, rph, status, UMMA_WAIT_FULL_TIMEOUT)) return false;
       const int g_last = (kdone + 35) >> 5;
-      if (seen_empty) ++acquired;
-      while (acquired <= g_last) {
-        if (!warp_wait(lane0, a_empty0 + 8 * (acquired & (kConvAStages - 1)), (uint32_t)((acquired / kConvAStages) & 1) ^ 1u, status,
-                       UMMA_WAIT_EMPTY_TIMEOUT))
-          return false;
-        ++acquired;
-      }
-      tc_fence_after();   // the MMAs that read these stages have completed (their commit): they may be written again
+      const uint32_t a_bar = empty0 + 8 * (g_last & (kConvAStages - 1)), a_par = (uint32_t)((g_last / kConvAStages) & 1) ^ 1u;
+      const bool a_free = mbar_test(a_bar, a_par);
       const unsigned char *base = rawpix_p + rs * slot_pitch + (uint32_t)(4 * quad_in_slot) * plane4;
       uint32_t v[36];
 #pragma unroll
@@ -311,46 +359,38 @@ struct ConvUmmaTf32 {
             v[i + 1] = __float_as_uint(*reinterpret_cast<const float *>(row + 4));
             v[i + 2] = __float_as_uint(*reinterpret_cast<const float *>(row + 8));
           }
+          if (MASK) v[i] &= taps[3 * dy], v[i + 1] &= taps[3 * dy + 1], v[i + 2] &= taps[3 * dy + 2];
         }
       }
-      // a look at the next step's barriers while the reads are in flight: a wait costs 100-200 clocks even
-      // when its barrier has completed
       const uint32_t rs_old = rs;
       const bool slot_done = ++quad_in_slot == quads;
       if (slot_done) {
         quad_in_slot = 0;
         if (++rs == (uint32_t)nslots) rs = 0, rph ^= 1;
       }
-      bool e = false, f = false;
-      if (s + 1 < steps) {
-        f = slot_done && mbar_test(raw_full0 + 8 * rs, rph);
-        if (acquired <= (kdone + 36 + 35) >> 5)
-          e = mbar_test(a_empty0 + 8 * (acquired & (kConvAStages - 1)), (uint32_t)((acquired / kConvAStages) & 1) ^ 1u);
-      }
+      const bool raw_next = s + 1 < steps && slot_done && mbar_test(raw_full0 + 8 * rs, rph);
+      if (!__all_sync(0xffffffffu, a_free) && !warp_wait(lane == 0, a_bar, a_par, status, UMMA_WAIT_EMPTY_TIMEOUT)) return false;
+      tc_fence_after();   // the MMAs that read these stages have completed (their commit): they may be written again
       const uint32_t col = (uint32_t)kdone & 127u;
 #pragma unroll
       for (int q = 0; q < 9; ++q) tmem_st_32x4(a_row + ((col + 4u * q) & 127u), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-      seen_raw = __all_sync(0xffffffffu, f);
-      seen_empty = __all_sync(0xffffffffu, e);
+      raw_seen = __all_sync(0xffffffffu, raw_next);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      // one arrival per warp: the slot is free (its values were written), and so is every stage whose 32nd
-      // column this step wrote
+      // one arrival per warp and barrier, each by a lane of its own: stages whose 32nd column this step wrote, the slot
       const int done_before = kdone >> 5;
       kdone += 36;
-      const int done_after = kdone >> 5;
-      if (lane0) {
-        if (slot_done) mbar_arrive(raw_empty0 + 8 * rs_old);
-        for (int g = done_before; g < done_after; ++g) mbar_arrive(a_full0 + 8 * (g & (kConvAStages - 1)));
-      }
+      const bool stage = lane < 2 && done_before + lane < kdone >> 5;
+      if (stage || (lane == 2 && slot_done))
+        mbar_arrive(stage ? full0 + 8 * (uint32_t)((done_before + lane) & (kConvAStages - 1)) : raw_empty0 + 8 * rs_old);
     }
     if (quad_in_slot) {   // the tile's channels end inside a slot: it is free too, and the next tile starts in a fresh one
-      if (lane0) mbar_arrive(raw_empty0 + 8 * rs);
+      if (lane == 0) mbar_arrive(raw_empty0 + 8 * rs);
       quad_in_slot = 0;
       if (++rs == (uint32_t)nslots) rs = 0, rph ^= 1;
     }
-    walk.rs = rs, walk.rph = rph, walk.quad_in_slot = quad_in_slot, walk.kdone = kdone, walk.acquired = acquired;
+    walk.rs = rs, walk.rph = rph, walk.kdone = kdone;
     return true;
   }
 
@@ -375,17 +415,35 @@ struct ConvUmmaTf32 {
   // scheduler, nothing to hide a branch behind -- more than the copying.  A wait costs 100-200 clocks even
   // when its barrier has completed, so every K block looks at the next one's barriers without blocking
   // while its own reads are in flight, and the next K block waits only for what was not there yet.
+  //
+  // PLANES: the whole-plane form (conv_plane_staging) for 3 x 3 windows on images whose rows are no 16-byte
+  // multiples.  What differs: a slot's channels come as one untiled copy per image, a tile's pixels are counted
+  // over the batch, taps outside the image are masked, there is no offset table, a weight stage and an A stage
+  // share one pair of barriers (four stages of each: the MMA thread waits once and commits once per K block), and
+  // K may be split over the CTAs of a cluster (whole channels: slices of 32 channels = 9 K blocks), whose partial sums meet in
+  // split_planes below.  Before it these layers were gathered by 4-byte copies, bound by the copies' issue:
+  // 512 -> 512 on 7 x 7, 32 images, 123 -> 33 us; 256 -> 256 on 14 x 14, 32 images, 65 -> 38 us.  Bound now by a
+  // step's chain on the repack warps -- barrier, reads, tensor-memory store, arrival, about 950 clocks for 36 values
+  // of k (the MMAs take 290) -- which a second CTA on the SM overlaps to about 650.
+  template <bool PLANES>
   __device__ __forceinline__ static void run_staged(const Params &p, const TileCtx &c) {
     const int warp = c.tid >> 5, lane = c.tid & 31;
     const int quad = (threadIdx.x >> 5) & 3;
     const int tile_px = p.st.tile_px;
-    const int ohw = p.oh * p.ow, K = p.K, num_kb = K / kBK;   // staged: K is a whole number of K blocks
+    const int ohw = p.oh * p.ow;
+    const int split = PLANES ? p.split : 1, kslice = PLANES ? c.vblock % split : 0;
+    const int kb0 = PLANES ? kslice * p.kb_per_slice : 0;     // first K block of this CTA's slice
+    const int num_kb = PLANES ? min(p.kb_per_slice, p.K / kBK - kb0) : p.K / kBK;   // staged: K is a whole number of K blocks
+    const int K = num_kb * kBK;
     // The CTA's tiles: its block index, then every p.ctas-th one (tiles numbered pixel tile fastest, then
     // channel tile, then image; a grid of one CTA per tile makes a single pass).  The rings, their barriers'
     // phases and tensor memory live across tiles, so the loads of the next tile run under this tile's
     // epilogue, and only the first tile pays for the set-up and the first loads' latency.
-    const int px_tiles = (ohw + tile_px - 1) / tile_px, co_tiles = (p.co + kUmmaBM - 1) / kUmmaBM;
-    const int total_tiles = px_tiles * co_tiles * p.n, tile_step = p.ctas;
+    // (whole planes: pixels counted over the batch, one "image"; the CTAs of a cluster share a tile)
+    const int co_tiles = (p.co + kUmmaBM - 1) / kUmmaBM, all_px = PLANES ? p.n * ohw : ohw;
+    const int px_tiles = (all_px + tile_px - 1) / tile_px;
+    const int total_tiles = px_tiles * co_tiles * (PLANES ? 1 : p.n), tile_step = PLANES ? p.ctas / split : p.ctas;
+    const int first_tile = PLANES ? c.vblock / split : c.vblock;
     const int wstages = p.stages;                             // 16 KB weight stages behind the raw ring
     int *const status = c.status;
     const uint32_t idesc = umma_idesc(0, kUmmaBM);            // M = 128 pixels, N = 128 output channels
@@ -396,7 +454,8 @@ struct ConvUmmaTf32 {
     const uint32_t raw_full0 = full0 + kConvRawBarOffset, raw_empty0 = raw_full0 + 8 * kConvMaxRawSlots;
     const uint32_t a_full0 = raw_empty0 + 8 * kConvMaxRawSlots, a_empty0 = a_full0 + 8 * kConvAStages;
     const uint32_t acc_empty = a_empty0 + 8 * kConvAStages;   // the epilogue has read the accumulator: the next tile's MMAs may start
-    const uint32_t raw0 = smem_u32(c.smem) + conv_header_bytes(K);
+    const uint32_t recv_bar = acc_empty + 8;                  // counts partial sums delivered by the cluster
+    const uint32_t raw0 = smem_u32(c.smem) + (PLANES ? kUmmaHeaderBytes : conv_header_bytes(K));
     const uint32_t wring = raw0 + (uint32_t)conv_raw_bytes(p.st.slots, p.st.slot_pitch);
     if (warp == 5) {
       if (!c.tmem_given) {   // (a persistent CTA of the work queue holds its columns already)
@@ -411,10 +470,10 @@ struct ConvUmmaTf32 {
     mark(MARK_START, c.tid == 0);
     if (warp == 4) {
       if (lane < wstages) {
-        mbar_init(full0 + 8 * lane, 1);    // the weight load's arrive.expect_tx
+        mbar_init(full0 + 8 * lane, PLANES ? 5 : 1);    // the weight load's arrive.expect_tx (and one arrival per repack warp)
         mbar_init(empty0 + 8 * lane, 1);   // the MMA's commit
       }
-      if (lane < kConvAStages) {
+      if (!PLANES && lane < kConvAStages) {
         mbar_init(a_full0 + 8 * lane, 4);  // one arrival per repack warp
         mbar_init(a_empty0 + 8 * lane, 1); // the MMA's commit
       }
@@ -425,16 +484,22 @@ struct ConvUmmaTf32 {
       if (lane == 0) {
         mbar_init(acc_bar, 1);
         mbar_init(acc_empty, 4);   // one arrival per epilogue warp
+        if (PLANES) mbar_init(recv_bar, 1);
       }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_w) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_x) : "memory");
+        if (!PLANES) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_x) : "memory");
+        if (PLANES && split > 1) {
+          int owned = 0;
+          for (int g = kslice; g < 8; g += split) ++owned;
+          mbar_expect_tx(recv_bar, (uint32_t)(owned * split) * (uint32_t)kConvGroupBytes);
+        }
       }
     }
     int *tab4 = reinterpret_cast<int *>(c.smem + kUmmaHeaderBytes);
-    if (warp < 4) {
+    if (!PLANES && warp < 4) {
       // entry k: the byte offset of (channel within its slot, dy, dx) inside a raw slot.  Thread t fills
       // entries t, t + 128, ...: (channel, tap) advance by the decomposition of 128, and tap -> (dy, dx)
       // is a multiply-shift (exact for taps < 32), so the loop has no division.
@@ -456,6 +521,9 @@ struct ConvUmmaTf32 {
     const uint32_t tmem_acc = c.tmem_given ? c.tmem_base : *reinterpret_cast<volatile uint32_t *>(tmem_slot);
     const uint32_t tmem_row = tmem_acc + ((uint32_t)(quad * 32) << 16);   // this warp's lanes; columns 0-127: accumulator, then the A stages
     mark(MARK_SETUP_DONE, c.tid == 0);
+    float *yp_split = nullptr;   // k-sliced planes: this lane's pixel of output channel 0 of the tile, channels left, accumulator ready
+    int co_split = 0;
+    bool acc_ok_split = false;
 
     if (warp == 4) {
       if (elect_one()) {
@@ -464,10 +532,22 @@ struct ConvUmmaTf32 {
         const int g_end = (K - 1) / kslot + 1;
         uint32_t rs = 0, rph = 1;
         bool ok = true;
-        for (int t = c.vblock; t < total_tiles && ok; t += tile_step) {
-          const int px0 = (t % px_tiles) * tile_px, img = t / (px_tiles * co_tiles);
+        for (int t = first_tile; t < total_tiles && ok; t += tile_step) {
+          const int px0 = (t % px_tiles) * tile_px, img = PLANES ? px0 / ohw : t / (px_tiles * co_tiles);
           const int y_start = (px0 / p.ow) * p.stride - p.pad;
+          const int imgs = PLANES ? (min(px0 + tile_px, all_px) - 1) / ohw - img + 1 : 1;
+          const size_t plane = (size_t)p.h * p.wd, img_stride = p.ci * plane;
+          const float *src = p.x + img * img_stride + (size_t)(kb0 * kBK / 9) * plane;   // PLANES: the slice's first channel
           for (int g = 0; g < g_end; ++g) {
+            if (PLANES) {
+              if (!(ok = mbar_wait(raw_empty0 + 8 * rs, rph, status, UMMA_WAIT_EMPTY_TIMEOUT))) break;
+              mbar_expect_tx(raw_full0 + 8 * rs, slot_bytes * (uint32_t)imgs);
+              for (int i = 0; i < imgs; ++i)
+                bulk_load(raw0 + rs * slot_pitch + (uint32_t)i * slot_bytes, src + i * img_stride, slot_bytes, raw_full0 + 8 * rs);
+              src += cc * plane;
+              if (++rs == (uint32_t)nslots) rs = 0, rph ^= 1;
+              continue;
+            }
             if (!(ok = mbar_wait(raw_empty0 + 8 * rs, rph, status, UMMA_WAIT_EMPTY_TIMEOUT))) break;
             mbar_expect_tx(raw_full0 + 8 * rs, slot_bytes);
             tma_load_4d(raw0 + rs * slot_pitch, &p.map_x, raw_full0 + 8 * rs, x_start, y_start, g * cc, img);
@@ -480,12 +560,12 @@ struct ConvUmmaTf32 {
       if (elect_one()) {
         uint32_t s = 0, ph = 1, dst = wring, bar = full0;
         bool ok = true;
-        for (int t = c.vblock; t < total_tiles && ok; t += tile_step) {
+        for (int t = first_tile; t < total_tiles && ok; t += tile_step) {
           const int co0 = (t / px_tiles % co_tiles) * kUmmaBM;
           for (int kb = 0; kb < num_kb; ++kb) {
             if (!(ok = mbar_wait(empty0 + 8 * s, ph, status, UMMA_WAIT_EMPTY_TIMEOUT))) break;
             mbar_expect_tx(bar, kUmmaABytes);
-            tma_load_3d(dst, &p.map_w, bar, kb * kBK, co0, 0);
+            tma_load_3d(dst, &p.map_w, bar, (kb0 + kb) * kBK, co0, 0);
             if (++s == (uint32_t)wstages) s = 0, ph ^= 1, dst = wring, bar = full0;
             else dst += kUmmaABytes, bar += 8;
           }
@@ -498,13 +578,13 @@ struct ConvUmmaTf32 {
         uint32_t s = 0, ph = 0, lo = lo0, as = 0, aph = 0;
         bool ok = true;
         int done = 0;   // K blocks issued so far, over all tiles
-        for (int t = c.vblock, it = 0; t < total_tiles && ok; t += tile_step, ++it) {
+        for (int t = first_tile, it = 0; t < total_tiles && ok; t += tile_step, ++it) {
           // the accumulator is free again once the epilogue of the tile before has read it
           if (it > 0 && !(ok = mbar_wait(acc_empty, (uint32_t)(it - 1) & 1u, status, UMMA_WAIT_ACC_TIMEOUT))) break;
           tc_fence_after();
           uint32_t accumulate = 0;
           for (int kb = 0; kb < num_kb; ++kb) {
-            ok = mbar_wait(a_full0 + 8 * as, aph, status, UMMA_WAIT_FULL_TIMEOUT) && mbar_wait(full0 + 8 * s, ph, status, UMMA_WAIT_FULL_TIMEOUT);
+            ok = (PLANES || mbar_wait(a_full0 + 8 * as, aph, status, UMMA_WAIT_FULL_TIMEOUT)) && mbar_wait(full0 + 8 * s, ph, status, UMMA_WAIT_FULL_TIMEOUT);
             if (!ok) break;
             tc_fence_after();
             if (kb == 0 && it == 0) mark(MARK_FIRST_FULL, true);
@@ -515,7 +595,7 @@ struct ConvUmmaTf32 {
               accumulate = 1;
             }
             umma_commit(empty0 + 8 * s);
-            umma_commit(a_empty0 + 8 * as);
+            if (!PLANES) umma_commit(a_empty0 + 8 * as);
             if (++s == (uint32_t)wstages) s = 0, ph ^= 1, lo = lo0;
             else lo += (uint32_t)kUmmaABytes >> 4;
             if (++as == (uint32_t)kConvAStages) as = 0, aph ^= 1;
@@ -527,7 +607,7 @@ struct ConvUmmaTf32 {
         // every commit has arrived before the barriers are invalidated and the ring is given up
         for (int j = max(0, done - wstages); j < done && ok; ++j)
           ok = mbar_wait(empty0 + 8 * (j % wstages), (uint32_t)(j / wstages) & 1u, status, UMMA_WAIT_EMPTY_TIMEOUT);
-        for (int j = max(0, done - kConvAStages); j < done && ok; ++j)
+        for (int j = max(0, done - kConvAStages); j < done && ok && !PLANES; ++j)
           ok = mbar_wait(a_empty0 + 8 * (j % kConvAStages), (uint32_t)(j / kConvAStages) & 1u, status, UMMA_WAIT_EMPTY_TIMEOUT);
       }
       __syncwarp();
@@ -555,23 +635,43 @@ struct ConvUmmaTf32 {
       // next k, how many slots from there on have been seen full, the A stage and its phase.
       int ahead = 0;
       uint32_t rs = 0, rph = 0, as = 0, aph = 1;
-      for (int t = c.vblock, it = 0; t < total_tiles && ok; t += tile_step, ++it) {
-        const int px0 = (t % px_tiles) * tile_px, co0 = (t / px_tiles % co_tiles) * kUmmaBM, img = t / (px_tiles * co_tiles);
-        const int pix = px0 + r;
-        // a lane past the tile's pixels or past the image reads the window of pixel 0 of the tile: finite
-        // values, and it is not stored
-        const int oy0 = px0 / ow;
-        int oy = pix / ow, ox = pix - oy * ow;
-        if (r >= tile_px || pix >= ohw) oy = oy0, ox = px0 - oy0 * ow;
-        const uint32_t rawpix = raw0 + (uint32_t)(((oy - oy0) * st.step_y * st.pitch + ox * st.step_x + st.x_off) * 4);
-        if (by_slot) {
+      for (int t = first_tile, it = 0; t < total_tiles && ok; t += tile_step, ++it) {
+        const int px0 = (t % px_tiles) * tile_px, co0 = (t / px_tiles % co_tiles) * kUmmaBM;
+        int img = PLANES ? px0 / ohw : t / (px_tiles * co_tiles), pix = px0 + r;
+        const bool live = r < tile_px && pix < all_px;
+        uint32_t taps[9];
+        uint32_t rawpix;
+        if (PLANES) {
+          // pixel of the batch -> image and pixel in it; a lane past the batch reads the tile's first pixel's window
+          const int at = live ? pix : px0, img0 = img;
+          img = at / ohw, pix = at - img * ohw;
+          const int oy = pix / ow, ox = pix - oy * ow, iy = oy * st.step_y + st.x_off, ix = ox * st.step_x + st.x_off;
+          rawpix = raw0 + (uint32_t)((img - img0) * st.slot_bytes + (iy * st.pitch + ix) * 4);
+#pragma unroll
+          for (int i = 0; i < 9; ++i)
+            taps[i] = (unsigned)(iy + i / 3) < (unsigned)st.rows && (unsigned)(ix + i % 3) < (unsigned)st.pitch ? 0xffffffffu : 0u;
+        } else {
+          // a lane past the tile's pixels or past the image reads the window of pixel 0 of the tile: finite
+          // values, and it is not stored
+          const int oy0 = px0 / ow;
+          int oy = pix / ow, ox = pix - oy * ow;
+          if (!live) oy = oy0, ox = px0 - oy0 * ow;
+          rawpix = raw0 + (uint32_t)(((oy - oy0) * st.step_y * st.pitch + ox * st.step_x + st.x_off) * 4);
+        }
+        if (PLANES) {
+          const unsigned char *const rawpix_p = conv_window + (int)(rawpix - smem_u32(conv_window));
+          // (rows of an odd width start at odd floats)
+          ok = pair && (st.pitch & 1) == 0
+                   ? repack_3x3<true, true>(c, K, rawpix_p, slot_pitch, nslots, st.cc / 4, plane4, pitch4, a_row, raw_full0, raw_empty0, full0, empty0, walk, taps)
+                   : repack_3x3<false, true>(c, K, rawpix_p, slot_pitch, nslots, st.cc / 4, plane4, pitch4, a_row, raw_full0, raw_empty0, full0, empty0, walk, taps);
+        } else if (by_slot) {
           const unsigned char *const rawpix_p = conv_window + (rawpix - smem_u32(conv_window));
-          ok = pair ? repack_3x3<true>(c, K, lane0, rawpix_p, slot_pitch, nslots, st.cc / 4, plane4, pitch4, a_row, raw_full0, raw_empty0, a_full0, a_empty0, walk)
-                    : repack_3x3<false>(c, K, lane0, rawpix_p, slot_pitch, nslots, st.cc / 4, plane4, pitch4, a_row, raw_full0, raw_empty0, a_full0, a_empty0, walk);
+          ok = pair ? repack_3x3<true, false>(c, K, rawpix_p, slot_pitch, nslots, st.cc / 4, plane4, pitch4, a_row, raw_full0, raw_empty0, a_full0, a_empty0, walk, taps)
+                    : repack_3x3<false, false>(c, K, rawpix_p, slot_pitch, nslots, st.cc / 4, plane4, pitch4, a_row, raw_full0, raw_empty0, a_full0, a_empty0, walk, taps);
         }
         int kin = 0;   // where the K block starts inside slot rs
         bool seen_empty = false, seen_raw = false;
-        for (int kb = 0; kb < num_kb && !by_slot; ++kb) {
+        for (int kb = 0; kb < num_kb && !PLANES && !by_slot; ++kb) {
           // one lane per warp polls a barrier and the warp follows it (its lanes meet again at the __syncwarp
           // before the arrival below, so the outcome of a wait has to be the same for all of them anyway)
           if (!seen_empty && !(ok = warp_wait(lane0, a_empty0 + 8 * as, aph, status, UMMA_WAIT_EMPTY_TIMEOUT))) break;
@@ -657,8 +757,11 @@ struct ConvUmmaTf32 {
           break;
         }
         float *const yp = y + ((size_t)img * co_total + co0) * ohw + pix;
-        const bool live = r < tile_px && pix < ohw;
         const int co_left = co_total - co0;
+        if (PLANES && split > 1) {   // this slice's share of the sum: the CTAs of the cluster meet below, with every thread
+          yp_split = live ? yp : nullptr, co_split = co_left, acc_ok_split = true;
+          continue;
+        }
 #pragma unroll 1
         for (int cc = 0; cc < kUmmaBM; cc += 32) {
           uint32_t r0[16], r1[16];
@@ -690,6 +793,7 @@ struct ConvUmmaTf32 {
         }
       }
     }
+    if (PLANES && split > 1) split_planes(c, split, kslice, ohw, raw0, recv_bar, tmem_row, acc_ok_split, yp_split, co_split);
     tc_fence_before();
     c.sync();
     if (warp == 5 && !c.tmem_given) tmem_dealloc(tmem_acc, kConvTmemCols);
@@ -698,7 +802,7 @@ struct ConvUmmaTf32 {
         mbar_inval(full0 + 8 * c.tid);
         mbar_inval(empty0 + 8 * c.tid);
       }
-      if (c.tid < kConvAStages) {
+      if (!PLANES && c.tid < kConvAStages) {
         mbar_inval(a_full0 + 8 * c.tid);
         mbar_inval(a_empty0 + 8 * c.tid);
       }
@@ -709,14 +813,66 @@ struct ConvUmmaTf32 {
       if (c.tid == 0) {
         mbar_inval(acc_bar);
         mbar_inval(acc_empty);
+        if (PLANES) mbar_inval(recv_bar);
       }
     }
     mark(MARK_END, c.tid == 0);
   }
 
+  // Not inlined: a third form inside run() cost the other two 1 % (batch-256 ResNet branch pair 149.9 -> 151.7 us).
+  __device__ __noinline__ static void run_planes(const Params &p, const TileCtx c) { run_staged<true>(p, c); }
+
+  // The sum over the k-slices of a tile whose accumulators hold pixels in their lanes and output channels in
+  // their columns; called by every thread of every CTA of the cluster after the MMAs.  The eight 16-channel
+  // groups are dealt to the slices round-robin; once the cluster has met (every MMA of the tile is done, so both
+  // rings are free) each CTA pushes its partial sums of a group into the owner's rings, [4-channel quarter]
+  // [pixel][4 floats], and the owner adds the slices in their order and stores 32 consecutive pixels a warp.
+  __device__ __forceinline__ static void split_planes(const TileCtx &c, int split, int kslice, int ohw, uint32_t ring, uint32_t recv_bar,
+                                                      uint32_t tmem_row, bool acc_ok, float *yp, int co_left) {
+    cluster_sync_all();
+    const int row = c.tid;   // the four repack warps: pixel = lane of tensor memory (quad * 32 + lane)
+    if (row >= kUmmaBM) return;
+    const int px = ((threadIdx.x >> 5) & 3) * 32 + (threadIdx.x & 31);
+    if (acc_ok) {
+#pragma unroll 1
+      for (int g = 0; g < 8; ++g) {
+        uint32_t r[16];
+        tmem_ld_32x16(tmem_row + g * 16, r);
+        tmem_ld_wait();
+        const uint32_t owner = (uint32_t)(g % split);
+        const uint32_t dst = peer_smem(ring + (uint32_t)((g / split) * split + kslice) * (uint32_t)kConvGroupBytes + (uint32_t)px * 16u, owner);
+        const uint32_t bar = peer_smem(recv_bar, owner);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) st_async_u4(dst + (uint32_t)(j * kUmmaBM * 16), bar, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+      }
+    }
+    if (!mbar_wait(recv_bar, 0, c.status, UMMA_WAIT_PEERS_TIMEOUT)) return;
+#pragma unroll 1
+    for (int g = kslice, li = 0; g < 8; g += split, ++li) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int s = 0; s < split; ++s) {
+          const float4 v = ld_shared_f4(ring + (uint32_t)(li * split + s) * (uint32_t)kConvGroupBytes + (uint32_t)((j * kUmmaBM + px) * 16));
+          a.x += v.x, a.y += v.y, a.z += v.z, a.w += v.w;
+        }
+        const int ch = g * 16 + 4 * j;
+        if (yp) {
+          float *q = yp + (size_t)ch * ohw;
+          if (ch < co_left) q[0] = a.x;
+          if (ch + 1 < co_left) q[ohw] = a.y;
+          if (ch + 2 < co_left) q[2 * (size_t)ohw] = a.z;
+          if (ch + 3 < co_left) q[3 * (size_t)ohw] = a.w;
+        }
+      }
+    }
+  }
+
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
     if (p.st.slots > 0) {
-      run_staged(p, c);
+      if (p.plane_imgs > 0) run_planes(p, c);
+      else run_staged<false>(p, c);
       return;
     }
     const int warp = c.tid >> 5, lane = c.tid & 31;

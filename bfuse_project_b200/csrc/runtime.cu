@@ -165,6 +165,17 @@ void pick_tile(int batch, int M, int N, int K, int elem, int sm_count, int share
 }
 
 int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *err) {
+// k-slices of a conv staged as whole planes: they hold whole groups of 32 channels (9 K blocks), none empty, and
+// 1, 2, 4 or 8 of them share the tile's eight 16-channel groups evenly
+bool plane_split_ok(int split, int ci) {
+  const int units = ci / 32;
+  return (split == 1 || split == 2 || split == 4 || split == 8) && (split - 1) * ceil_div(units, split) < units;
+}
+// The runtime's own choice is 1 or 4, as for every operator (a fused launch has one cluster width): 4 while the
+// slices fit the two CTAs an SM holds (512 -> 512 on 7 x 7, 32 images, 52 tiles: 70 us with one slice, 33 with
+// four; 256 -> 256 on 14 x 14, 32 images, 98 tiles: 38 us with one, 40 with four).
+int plane_split(int tiles, int ci, int share, int sm) { return (long long)tiles * 4 * share <= 2 * sm && plane_split_ok(4, ci) ? 4 : 1; }
+
   const int *s = d->shape;
   auto set = [&](int gx, int gy, int gz, int bx, int by, size_t smem, int nargs) {
     d->GridDim = {gx, gy, gz};
@@ -219,6 +230,33 @@ int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *
       if (oh <= 0 || ow <= 0) { *err = "conv2d: empty output"; return BFUSE_ERR_SHAPE; }
       const int num_kb = ceil_div(s[1] * s[5] * s[6], ConvUmmaTf32::kBK);
       // pixels per tile: the widest of 128 / 64 / 32 that still gives the operator about half the
+      // Whole planes, shape[11] = 3: 3 x 3 windows on images whose rows the TMA cannot describe, once the batch holds
+      // a whole 128-pixel tile and the gathered form's 32-pixel tiles, split four ways, no longer find an SM each.
+      // Alone, gathered against planes: 512 -> 512 on 7 x 7, 4 images (128 such CTAs) 23.7 / 25.1 us, 8 images
+      // 63 / 25 us, 32 images 123 / 33 us; 256 -> 256 on 14 x 14, 3 images (168 CTAs) 18.5 / 16.9, 32 images 65 / 38 us;
+      // 256 -> 512 with stride 2, 4 images 16.0 / 18.0, 32 images 45 / 24 us.
+      ConvStaging rows, planes;
+      const long long gathered_ctas = 4LL * s[0] * ceil_div(oh * ow, 32) * ceil_div(s[4], kUmmaBM);
+      if (s[11] == 3 || (s[11] == 0 && s[9] <= 0 && s[10] <= 0 && (long long)s[0] * oh * ow >= kConvBN && gathered_ctas * share > sm &&
+                         !conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, kConvBN, &rows))) {
+        const int imgs = conv_plane_staging(s[0], s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, &planes);
+        if (!imgs && s[11] == 3) { *err = "conv2d: shape[11] = 3 (whole planes) needs a 3 x 3 window, ci a multiple of 32 and four planes of a tile's images in 16 KB"; return BFUSE_ERR_SHAPE; }
+        if (imgs) {
+          const int px_tiles = ceil_div(s[0] * oh * ow, planes.tile_px), co_tiles = ceil_div(s[4], kUmmaBM), tiles = px_tiles * co_tiles;
+          int split = s[10];
+          if (split <= 0) split = plane_split(tiles, s[1], share, sm);
+          if (!plane_split_ok(split, s[1]) || (s[9] > 0 && s[9] != kConvBN)) { *err = "conv2d: shape[11] = 3 (whole planes) takes 128-pixel tiles and 1, 2, 4 or 8 k-slices of whole groups of 32 channels"; return BFUSE_ERR_SHAPE; }
+          const int Kslice = ceil_div(s[1] / 32, split) * 288;
+          // two CTAs per SM, whatever the grid
+          planes.slots = conv_plane_slots(110 * 1024, Kslice, planes.cc, planes.slot_pitch);
+          if (!planes.slots) { *err = "conv2d: shape[11] = 3 (whole planes): the raw ring does not fit the shared-memory budget"; return BFUSE_ERR_SHAPE; }
+          d->shape[9] = kConvBN, d->shape[10] = split, d->shape[11] = 3;
+          const int smem = conv_staged_smem_bytes(kUmmaHeaderBytes, planes.slots, planes.slot_pitch, kConvAStages);
+          if (split == 1 && tiles > 2 * sm) set(2 * sm, 1, 1, kConvThreads, 1, smem, 3);   // (as for staged rows below)
+          else set(split * px_tiles, co_tiles, 1, kConvThreads, 1, smem, 3);
+          return BFUSE_OK;
+        }
+      }
       // SMs (its pair partner takes the other half); a single small image gets 32-pixel tiles
       int bn = s[9];
       if (bn <= 0 && s[11] == 1) bn = kConvBN;   // the staged form has one tile: the 128 lanes of tensor memory
@@ -257,7 +295,7 @@ int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *
         return BFUSE_ERR_SHAPE;
       }
       if (s[11] == 0 && split == 1 && !conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, bn, &st)) st.slots = 0;
-      if (s[11] < 0 || s[11] > 2) { *err = "conv2d: shape[11] (operand mode) must be 0, 1 or 2"; return BFUSE_ERR_SHAPE; }
+      if (s[11] < 0 || s[11] > 3) { *err = "conv2d: shape[11] (operand mode) must be 0, 1, 2 or 3"; return BFUSE_ERR_SHAPE; }
       d->shape[11] = st.slots ? 1 : 2;
       // ring budget: the whole SM when the operator and an equal partner leave every CTA an SM of its own, else
       // two CTAs per SM (staged: tensor memory holds two) or three (gathered)
@@ -275,9 +313,9 @@ int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *
         // walk their whole share of the tiles, alone.
         const long long staged_tiles = (long long)ceil_div(oh * ow, st.tile_px) * ceil_div(s[4], kUmmaBM) * s[0];
         if (staged_tiles > 2 * sm)
-          set(2 * sm, 1, 1, kConvThreads, 1, conv_staged_smem_bytes(K, st.slots, st.slot_pitch, wst), 3);
+          set(2 * sm, 1, 1, kConvThreads, 1, conv_staged_smem_bytes(conv_header_bytes(K), st.slots, st.slot_pitch, wst), 3);
         else
-          set(ceil_div(oh * ow, st.tile_px), ceil_div(s[4], kUmmaBM), s[0], kConvThreads, 1, conv_staged_smem_bytes(K, st.slots, st.slot_pitch, wst), 3);
+          set(ceil_div(oh * ow, st.tile_px), ceil_div(s[4], kUmmaBM), s[0], kConvThreads, 1, conv_staged_smem_bytes(conv_header_bytes(K), st.slots, st.slot_pitch, wst), 3);
         return BFUSE_OK;
       }
       int stages = std::max(1, std::min({q, kUmmaMaxStages, (budget - conv_header_bytes(K)) / conv_stage_bytes(bn)}));
@@ -480,11 +518,20 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
       if (kd.bx != kConvThreads || kd.by != 1 || kd.bz != 1) return shape_err("BlockDim must be (224, 1, 1)");
       const int bn = s[9] > 0 ? s[9] : kConvBN;
       if (bn != 32 && bn != 64 && bn != 128) return shape_err("shape[9] (pixels per tile) must be 32, 64 or 128");
-      const int split = s[10] > 0 ? s[10] : 1, num_kb = ceil_div(K, ConvUmmaTf32::kBK), q = ceil_div(num_kb, split);
+      ConvStaging planes;
+      const int plane_imgs = s[11] == 3 ? conv_plane_staging(s[0], s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, &planes) : 0;
+      if (s[11] == 3 && (!plane_imgs || bn != kConvBN || !plane_split_ok(s[10] > 0 ? s[10] : 1, s[1])))
+        return shape_err("shape[11] = 3 (whole planes) needs a 3 x 3 window, ci a multiple of 32, four planes of a tile's images in 16 KB, 128-pixel tiles and 1, 2, 4 or 8 k-slices of whole groups of 32 channels");
+      const int split = s[10] > 0 ? s[10] : 1, num_kb = ceil_div(K, ConvUmmaTf32::kBK);
+      const int q = plane_imgs ? ceil_div(s[1] / 32, split) * 9 : ceil_div(num_kb, split);
       if (split > 8 || (split - 1) * q >= num_kb) return shape_err("shape[10] (k-slices) must be 1..8 with every k-slice non-empty");
       ConvStaging geometry;   // a staged conv's tiles may be whole output rows: fewer than BN pixels
       const int tile_px = s[11] == 1 && conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, bn, &geometry) ? geometry.tile_px : bn;
-      if (s[11] == 1) {
+      if (plane_imgs) {
+        const int px_tiles = ceil_div(s[0] * oh * ow, planes.tile_px), co_tiles = ceil_div(s[4], kUmmaBM);
+        if (split > 1 ? (kd.gx != split * px_tiles || kd.gy != co_tiles || kd.gz != 1) : (long long)kd.gx * kd.gy * kd.gz > (long long)px_tiles * co_tiles)
+          return shape_err("GridDim of a conv staged as whole planes must be (k-slices * ceil(n*oh*ow / 128), ceil(co/128), 1), or hold fewer CTAs with one k-slice");
+      } else if (s[11] == 1) {
         if ((long long)kd.gx * kd.gy * kd.gz > (long long)ceil_div(oh * ow, tile_px) * ceil_div(s[4], kUmmaBM) * s[0])
           return shape_err("GridDim of a staged conv must not hold more CTAs than the conv has tiles (a CTA takes every grid-size-th tile)");
       } else if (kd.gx != split * ceil_div(oh * ow, tile_px) || kd.gy != ceil_div(s[4], kUmmaBM) || kd.gz != s[0]) {
@@ -498,11 +545,19 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
       // else gathered from global memory.  The raw ring is 3 slots deep, 4 when room is left for a
       // whole-SM operand ring as well.
       const int min_stages = ceil_div(umma_epilogue_bytes(bn, split, 4), conv_stage_bytes(bn));
-      if (s[11] < 0 || s[11] > 2) return shape_err("shape[11] (operand mode) must be 0 (the runtime's choice), 1 (staged) or 2 (gathered)");
+      if (s[11] < 0 || s[11] > 3) return shape_err("shape[11] (operand mode) must be 0 (the runtime's choice), 1 (staged), 2 (gathered) or 3 (whole planes)");
       if (s[11] == 1 && (split != 1 || !conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, bn, &p.st)))
         return shape_err("shape[11] = 1 (staged operand) needs 128-pixel tiles, an unsplit K of whole K blocks, image rows of 16-byte multiples and a window whose rows fit a 24 KB slot");
       int wstages = 0;
-      if (s[11] == 1) {
+      if (plane_imgs) {
+        p.st = planes;
+        p.plane_imgs = plane_imgs;
+        p.st.slots = conv_plane_slots((int)std::min<size_t>(k.smem, kMaxSmemPerCta), q * ConvUmmaTf32::kBK, planes.cc, planes.slot_pitch);
+        wstages = kConvAStages;
+        if (!p.st.slots || k.smem < (size_t)conv_staged_smem_bytes(kUmmaHeaderBytes, p.st.slots, planes.slot_pitch, wstages))
+          return shape_err("shape[11] = 3 (whole planes): shared memory below the raw ring plus four weight stages");
+        static_assert(kConvAStages * kUmmaABytes >= conv_plane_recv_bytes(8), "the k-slices' sums fit the weight stages");
+      } else if (s[11] == 1) {
         if (!conv_staged_ring((int)std::min<size_t>(k.smem, kMaxSmemPerCta), K, p.st.cc * s[5] * s[6], p.st.slot_pitch, &p.st.slots, &wstages))
           return shape_err("shape[11] = 1 (staged operand): shared memory below the raw ring plus two weight stages");
       } else if (k.smem < (size_t)conv_umma_smem_bytes(min_stages, bn, K, 0)) {
@@ -510,7 +565,7 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
       }
       int rc = encode_map(ctx, &p.map_w, 4, a[1], K, s[4], 1, kUmmaBM);
       if (rc) return rc;
-      if (p.st.slots) {
+      if (p.st.slots && !plane_imgs) {
         // the NCHW input as {w, h, ci, n}; a box is one slot: pitch x rows x cc elements, rows taken with element stride ey
         const cuuint64_t dims[4] = {(cuuint64_t)s[3], (cuuint64_t)s[2], (cuuint64_t)s[1], (cuuint64_t)s[0]};
         const cuuint64_t strides[3] = {(cuuint64_t)s[3] * 4, (cuuint64_t)s[3] * s[2] * 4, (cuuint64_t)s[3] * s[2] * s[1] * 4};
@@ -683,6 +738,7 @@ bool ring_info(const KernelRec &k, int *header, int *stage_bytes, int *min_stage
     const ConvUmmaParams *cp = reinterpret_cast<const ConvUmmaParams *>(k.params);
     const int K = s[1] * s[5] * s[6];
     if (cp->st.slots) {   // staged: the raw ring stays as registered, the 16 KB weight stages are what can be given up
+    if (cp->plane_imgs) return false;   // whole planes: weight and A stages share their barriers, four of each
       *header = conv_header_bytes(K) + conv_raw_bytes(cp->st.slots, cp->st.slot_pitch), *stage_bytes = kUmmaABytes;
       *min_stages = std::min(2, K / ConvUmmaTf32::kBK);
     } else {
@@ -974,7 +1030,7 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
   // tensor-memory columns an operator's CTA allocates
   auto tmem_cols = [](const KernelRec &k) {
     if (k.desc.op == BFUSE_OP_GEMM_TF32 || k.desc.op == BFUSE_OP_GEMM_BF16) return k.desc.shape[4] * std::max(1, k.desc.shape[6] / kUmmaBM);
-    if (k.desc.op == BFUSE_OP_CONV2D_TF32 && k.desc.shape[11] == 1) return kConvTmemCols;   // staged: accumulator and operand stages
+    if (k.desc.op == BFUSE_OP_CONV2D_TF32 && (k.desc.shape[11] & 1)) return kConvTmemCols;   // staged: accumulator and operand stages
     return k.desc.op == BFUSE_OP_CONV2D_TF32 ? (k.desc.shape[9] > 0 ? k.desc.shape[9] : kConvBN) : 0;
   };
   // a persistent CTA of the work queue allocates once what either operator's tile may need (a power of two >= 32)

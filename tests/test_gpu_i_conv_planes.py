@@ -1,0 +1,81 @@
+"""Convs staged as whole image planes (shape[11] = 3): 3 x 3 windows on images whose rows are no 16-byte multiples."""
+import numpy as np
+import pytest
+
+import bfuse_project_b200 as bf
+from bfuse_project_b200 import workloads as wl
+from test_gpu_b_pairs import BLOCK_PATTERNS, run_and_check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rt():
+    r = bf.Runtime(0)
+    yield r
+    r.close()
+
+
+# n, ci, h = w, co, stride, pad, k-slices
+SHAPES = [
+    (1, 32, 14, 40, 1, 1, 1),      # one image, a tile and a half; ragged channel tile
+    (3, 64, 7, 128, 1, 1, 2),      # a tile over three images, the second one partly filled; one group of channels a slice
+    (5, 128, 14, 136, 2, 1, 4),    # stride 2 on an even width (8-byte reads), tiles of whole images
+    (4, 256, 7, 130, 1, 1, 8),     # eight slices
+    (11, 64, 5, 128, 1, 0, 1),     # no padding: nine pixels an image, fifteen images a tile
+    (9, 96, 10, 64, 2, 2, 1),      # padding 2
+    (9, 96, 13, 64, 1, 2, 2),      # two slices of two and one channel groups
+]
+
+
+@pytest.mark.parametrize("n,ci,hw,co,stride,pad,split", SHAPES)
+def test_planes_against_the_oracle_and_unfused(rt, n, ci, hw, co, stride, pad, split):
+    """The tolerances are the tf32 conv's (pair_oracle); fused == unfused bit for bit."""
+    rng = np.random.default_rng(ci + hw)
+    a = wl.conv2d("planes", rng, bf.OP_CONV2D_TF32, n, ci, hw, hw, co, 3, stride, pad, bn=128, split=split, mode=3)
+    b = wl.gemm("g", rng, bf.OP_GEMM_TF32, 1, 100, 64, 64, w_std=1.0, bn=64, split=1)
+    run_and_check(rt, wl.PairSpec("planes", a, b, "tf32", "hbm"), BLOCK_PATTERNS if split == 1 else [(bf.ZIGZAG, 1, 1), (bf.RANGE_SPLIT, 0, 0)])
+    if split == 1:
+        run_and_check(rt, wl.PairSpec("planes_twice", a, a, "tf32", "hbm"), [(bf.WORK_QUEUE, 1, 1), (bf.THREAD_SPLIT, 0, 0)])
+
+
+def test_the_runtime_takes_planes_for_small_images_of_a_batch(rt):
+    def mode(n, ci, hw, co, flags=0):
+        d = rt.describe("c", bf.OP_CONV2D_TF32, (n, ci, hw, hw, co, 3, 3, 1, 1, 0, 0, 0), flags=flags)
+        return d.shape[11], d.shape[10]
+    assert mode(32, 512, 7, 512, bf.flag_share(1)) == (3, 4) and mode(32, 256, 14, 256, bf.flag_share(1)) == (3, 1)
+    assert mode(1, 512, 7, 512)[0] == 2 and mode(32, 128, 28, 128)[0] == 1      # a lone image; rows of 16-byte multiples
+
+
+def test_planes_that_cannot_be_are_rejected(rt):
+    for n, ci, hw, co, k, bn, split in ((4, 40, 7, 64, 3, 128, 1), (4, 64, 7, 64, 1, 128, 1), (4, 64, 7, 64, 3, 64, 1), (4, 64, 7, 64, 3, 128, 4), (4, 64, 62, 64, 3, 128, 1)):
+        with pytest.raises(bf.BfuseError) as err:
+            rt.describe("c", bf.OP_CONV2D_TF32, (n, ci, hw, hw, co, k, k, 1, k // 2, bn, split, 3))
+        assert err.value.code == 2
+
+
+def test_ctas_that_walk_several_tiles_and_values_outside_a_window(rt):
+    """A grid smaller than the tile count writes the same bits; an infinity reaches only the windows that hold it,
+    although a tap outside its image reads whatever lies beside the plane."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    n, ci, hw, co = 40, 32, 7, 136
+    x = torch.randn(n, ci, hw, hw, device="cuda", generator=g)
+    w = torch.randn(co, ci, 3, 3, device="cuda", generator=g) * 0.05
+    outs = []
+    for grid in (None, (3, 1, 1), (1, 1, 1)):
+        y = torch.zeros(n, co, hw, hw, device="cuda")
+        d = rt.describe("c", bf.OP_CONV2D_TF32, (n, ci, hw, hw, co, 3, 3, 1, 1, 128, 1, 3), [x.data_ptr(), w.data_ptr(), y.data_ptr()], grid=grid)
+        k = rt.register_kernel(d)
+        rt.launch_kernel(k)
+        assert rt.read_status() == 0
+        outs.append(y)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    x[1, 3, 0, 0] = float("inf")                     # a corner: the next row's end and the next image's start lie beside it
+    rt.launch_kernel(k)
+    assert rt.read_status() == 0
+    touched = torch.zeros(n, 1, hw, hw, dtype=torch.bool, device="cuda")
+    touched[1, 0, :2, :2] = True
+    assert torch.equal(outs[2][~touched.expand_as(outs[2])], outs[0][~touched.expand_as(outs[0])])
+    assert not torch.isfinite(outs[2][1, :, :2, :2]).any()

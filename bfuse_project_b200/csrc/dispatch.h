@@ -50,6 +50,8 @@ struct DispatchTable {
   int no_pdl;              // host side only: launch without the programmatic-dependent-launch attribute
   int tmem_cols;           // queue launches: tensor-memory columns a persistent CTA allocates ONCE for all its tickets
                            // (the larger need of the two operators, a power of two; 0: neither uses tensor memory)
+  int per_cta[2];          // > 1: a CTA runs that many consecutive virtual blocks of the operator, n_cta counting such
+  int n_block[2];          //      runs and n_block the operator's virtual blocks (0 or 1: one block a CTA)
 };
 
 // Dispatch unit (or ticket) b -> operator k and its virtual unit.  Returns false if b is unmapped.

@@ -47,9 +47,8 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
   return t;
 }
 
-template <class Op>
-__device__ __forceinline__ void run_tile(const typename Op::Params &p, const DispatchTable &t, int k, int vb, int vtid,
-                                         int bar_id, unsigned char *smem, int shares_cta = 0, int tmem_given = 0, unsigned tmem_base = 0) {
+__device__ __forceinline__ TileCtx tile_ctx(const DispatchTable &t, int k, int vb, int vtid, int bar_id, unsigned char *smem, int shares_cta = 0,
+                                            int tmem_given = 0, unsigned tmem_base = 0) {
   TileCtx c;
   c.vblock = vb;
   c.tid = vtid;
@@ -65,7 +64,37 @@ __device__ __forceinline__ void run_tile(const typename Op::Params &p, const Dis
   c.persistent = t.queue | shares_cta;
   c.tmem_given = tmem_given;
   c.tmem_base = tmem_base;
-  Op::run(p, c);
+  return c;
+}
+
+template <class Op>
+__device__ __forceinline__ void run_tile(const typename Op::Params &p, const DispatchTable &t, int k, int vb, int vtid,
+                                         int bar_id, unsigned char *smem, int shares_cta = 0, int tmem_given = 0, unsigned tmem_base = 0) {
+  Op::run(p, tile_ctx(t, k, vb, vtid, bar_id, smem, shares_cta, tmem_given, tmem_base));
+}
+
+// The virtual blocks of one CTA of an operator: block vb, or (RUNS: a memory-bound body beside one with tensor memory,
+// in the register-rich build of the pair) the t.per_cta[k] consecutive ones of run vb, Op::kRunRows at a time.  See
+// bfuse_register_fusion for when CTAs take runs.
+template <class Op, bool RUNS>
+__device__ __forceinline__ void run_blocks(const typename Op::Params &p, const DispatchTable &t, int k, int vb, int vtid,
+                                           int bar_id, unsigned char *smem, int tmem_given, unsigned tmem_base) {
+  if constexpr (RUNS) {
+    if (t.per_cta[k] > 1) {
+      const int end = min((vb + 1) * t.per_cta[k], t.n_block[k]);
+      for (int v = vb * t.per_cta[k]; v < end; v += Op::kRunRows) {
+        TileCtx c = tile_ctx(t, k, v, vtid, bar_id, smem);
+        if (v > vb * t.per_cta[k]) {
+          c.waited = 1;
+          c.sync();   // this block writes the same shared memory
+        }
+        if constexpr (Op::kRunRows > 1) Op::template run_rows<Op::kRunRows>(p, c, end);
+        else Op::run(p, c);
+      }
+      return;
+    }
+  }
+  run_tile<Op>(p, t, k, vb, vtid, bar_id, smem, 0, tmem_given, tmem_base);
 }
 
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
@@ -158,9 +187,9 @@ __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
       if (t.cta_times) t_body = global_timer_ns();
       // guard of the reference: KernelID_ == k && threadIdx.x < B_k (Algorithms.cc:699-717)
       if (k == 0) {
-        if (tid < t.n_thr[0]) run_tile<A>(pa, t, 0, vb, tid, 1, smem, 0, queue_tmem_cols > 0, queue_tmem);
+        if (tid < t.n_thr[0]) run_blocks<A, A::kMemoryBound && B::kUsesTmem && MINB == 2>(pa, t, 0, vb, tid, 1, smem, queue_tmem_cols > 0, queue_tmem);
       } else {
-        if (tid < t.n_thr[1]) run_tile<B>(pb, t, 1, vb, tid, 2, smem, 0, queue_tmem_cols > 0, queue_tmem);
+        if (tid < t.n_thr[1]) run_blocks<B, B::kMemoryBound && A::kUsesTmem && MINB == 2>(pb, t, 1, vb, tid, 2, smem, queue_tmem_cols > 0, queue_tmem);
       }
       if (t.cta_times && tid == 0) {  // kernel entry, body start (its set-up may overlap the previous kernel), thread 0 done
         t.cta_times[3 * (size_t)ticket] = t_entry;

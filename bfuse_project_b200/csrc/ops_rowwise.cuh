@@ -19,6 +19,7 @@ constexpr int kRowMaxVec = 4;  // 128-bit vectors a thread may hold per row (row
 
 // ---------------------------------------------------------------------------------- softmax
 struct SoftmaxF32 {
+  static constexpr int kRunRows = 2;   // blocks a CTA that takes runs of them works on at once (fused_block_kernel)
   struct Params {
     const float *x;
     float *y;
@@ -30,47 +31,69 @@ struct SoftmaxF32 {
   static constexpr bool kMemoryBound = true;
   static constexpr bool kUsesTmem = false;   // allocates tensor memory (see fused_block_kernel)
 
-  __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
+  __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) { run_rows<1>(p, c, c.vblock + 1); }
+
+  // R consecutive virtual blocks at once, c.vblock first and none at or past `end`: a thread has a row of each.
+  template <int R>
+  __device__ __forceinline__ static void run_rows(const Params &p, const TileCtx &c, int end) {
     c.dependency_wait();
-    const int tpr = c.bx, lane = c.tid % tpr, row = c.vblock * c.by + c.tid / tpr;
+    const int tpr = c.bx, lane = c.tid % tpr, row0 = c.vblock * c.by + c.tid / tpr;
     const int nvec = p.cols / (4 * tpr);
-    const bool live = row < p.rows;
-    const float4 *xr = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.cols);
-    float4 v[kRowMaxVec];
-    // every load of the row is issued before the first use of any of them: a use between two loads
+    float4 v[R][kRowMaxVec];
+    bool live[R];
+    // every load of the rows is issued before the first use of any of them: a use between two loads
     // would make the second one wait for the first one's trip to DRAM
 #pragma unroll
-    for (int i = 0; i < kRowMaxVec; ++i)
-      if (i < nvec && live) v[i] = ld_stream_f4(xr + i * tpr + lane);
-    float m = -INFINITY;
+    for (int r = 0; r < R; ++r) {
+      const int row = row0 + r * c.by;
+      live[r] = c.vblock + r < end && row < p.rows;
+      const float4 *xr = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.cols);
 #pragma unroll
-    for (int i = 0; i < kRowMaxVec; ++i) {
-      if (i < nvec && live) {
-        v[i].x *= p.scale, v[i].y *= p.scale, v[i].z *= p.scale, v[i].w *= p.scale;
-        m = fmaxf(m, fmaxf(fmaxf(v[i].x, v[i].y), fmaxf(v[i].z, v[i].w)));
+      for (int i = 0; i < kRowMaxVec; ++i)
+        if (i < nvec && live[r]) v[r][i] = ld_stream_f4(xr + i * tpr + lane);
+    }
+    float m[R], s[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      m[r] = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < kRowMaxVec; ++i) {
+        if (i < nvec && live[r]) {
+          float4 &a = v[r][i];
+          a.x *= p.scale, a.y *= p.scale, a.z *= p.scale, a.w *= p.scale;
+          m[r] = fmaxf(m[r], fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)));
+        }
       }
     }
-    m = row_reduce<OpMax>(m, c, tpr, 0);
+    row_reduce<OpMax, R>(m, c, tpr, 0);
     constexpr float kLog2e = 1.4426950408889634f;
-    float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < kRowMaxVec; ++i) {
-      if (i < nvec && live) {
-        v[i].x = exp2f((v[i].x - m) * kLog2e);
-        v[i].y = exp2f((v[i].y - m) * kLog2e);
-        v[i].z = exp2f((v[i].z - m) * kLog2e);
-        v[i].w = exp2f((v[i].w - m) * kLog2e);
-        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    for (int r = 0; r < R; ++r) {
+      s[r] = 0.f;
+#pragma unroll
+      for (int i = 0; i < kRowMaxVec; ++i) {
+        if (i < nvec && live[r]) {
+          float4 &a = v[r][i];
+          a.x = exp2f((a.x - m[r]) * kLog2e);
+          a.y = exp2f((a.y - m[r]) * kLog2e);
+          a.z = exp2f((a.z - m[r]) * kLog2e);
+          a.w = exp2f((a.w - m[r]) * kLog2e);
+          s[r] += (a.x + a.y) + (a.z + a.w);
+        }
       }
     }
-    s = row_reduce<OpSum>(s, c, tpr, 1);
-    const float inv = 1.f / s;
-    float4 *yr = reinterpret_cast<float4 *>(p.y + (size_t)row * p.cols);
+    row_reduce<OpSum, R>(s, c, tpr, 1);
 #pragma unroll
-    for (int i = 0; i < kRowMaxVec; ++i) {
-      if (i < nvec && live) {
-        v[i].x *= inv, v[i].y *= inv, v[i].z *= inv, v[i].w *= inv;
-        st_stream_f4(yr + i * tpr + lane, v[i]);
+    for (int r = 0; r < R; ++r) {
+      const float inv = 1.f / s[r];
+      float4 *yr = reinterpret_cast<float4 *>(p.y + (size_t)(row0 + r * c.by) * p.cols);
+#pragma unroll
+      for (int i = 0; i < kRowMaxVec; ++i) {
+        if (i < nvec && live[r]) {
+          float4 &a = v[r][i];
+          a.x *= inv, a.y *= inv, a.z *= inv, a.w *= inv;
+          st_stream_f4(yr + i * tpr + lane, a);
+        }
       }
     }
   }
@@ -78,6 +101,7 @@ struct SoftmaxF32 {
 
 // -------------------------------------------------------------------- (residual +) LayerNorm
 struct LayerNormF32 {
+  static constexpr int kRunRows = 1;
   struct Params {
     const float *x;
     const float *res;  // nullptr: plain LayerNorm
@@ -162,6 +186,7 @@ __device__ __forceinline__ uint32_t f2_to_bf16x2(float lo, float hi) {
 }
 
 struct RmsNormBf16 {
+  static constexpr int kRunRows = 1;
   struct Params {
     const uint16_t *x;
     const uint16_t *w;
@@ -226,6 +251,7 @@ struct RmsNormBf16 {
 // is 8 consecutive rotary pairs (dim / 16 chunks per head); a thread computes the 8 sin/cos of its
 // (position, chunk) once and applies them to heads / head_groups heads.
 struct RopeBf16 {
+  static constexpr int kRunRows = 1;
   struct Params {
     const uint16_t *q;
     const float *inv_freq;  // [dim / 2]

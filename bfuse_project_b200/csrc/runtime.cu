@@ -53,6 +53,7 @@ struct FusionRec {
   bool retiled[2];
   int users;            // live graphs that captured it
   FusedPlan plan;
+  DispatchTable launch;  // what the kernel decodes: plan.table, or the same pattern over runs of blocks (per_cta)
   std::string name;
   size_t smem;
   unsigned launch_grid;
@@ -164,7 +165,6 @@ void pick_tile(int batch, int M, int N, int K, int elem, int sm_count, int share
   *split_out = split_fixed > 0 ? split_fixed : best_split;
 }
 
-int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *err) {
 // k-slices of a conv staged as whole planes: they hold whole groups of 32 channels (9 K blocks), none empty, and
 // 1, 2, 4 or 8 of them share the tile's eight 16-channel groups evenly
 bool plane_split_ok(int split, int ci) {
@@ -176,6 +176,7 @@ bool plane_split_ok(int split, int ci) {
 // four; 256 -> 256 on 14 x 14, 32 images, 98 tiles: 38 us with one, 40 with four).
 int plane_split(int tiles, int ci, int share, int sm) { return (long long)tiles * 4 * share <= 2 * sm && plane_split_ok(4, ci) ? 4 : 1; }
 
+int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *err) {
   const int *s = d->shape;
   auto set = [&](int gx, int gy, int gz, int bx, int by, size_t smem, int nargs) {
     d->GridDim = {gx, gy, gz};
@@ -229,7 +230,6 @@ int plane_split(int tiles, int ci, int share, int sm) { return (long long)tiles 
       const int oh = conv_out(s[2], s[5], s[7], s[8]), ow = conv_out(s[3], s[6], s[7], s[8]);
       if (oh <= 0 || ow <= 0) { *err = "conv2d: empty output"; return BFUSE_ERR_SHAPE; }
       const int num_kb = ceil_div(s[1] * s[5] * s[6], ConvUmmaTf32::kBK);
-      // pixels per tile: the widest of 128 / 64 / 32 that still gives the operator about half the
       // Whole planes, shape[11] = 3: 3 x 3 windows on images whose rows the TMA cannot describe, once the batch holds
       // a whole 128-pixel tile and the gathered form's 32-pixel tiles, split four ways, no longer find an SM each.
       // Alone, gathered against planes: 512 -> 512 on 7 x 7, 4 images (128 such CTAs) 23.7 / 25.1 us, 8 images
@@ -257,6 +257,7 @@ int plane_split(int tiles, int ci, int share, int sm) { return (long long)tiles 
           return BFUSE_OK;
         }
       }
+      // pixels per tile: the widest of 128 / 64 / 32 that still gives the operator about half the
       // SMs (its pair partner takes the other half); a single small image gets 32-pixel tiles
       int bn = s[9];
       if (bn <= 0 && s[11] == 1) bn = kConvBN;   // the staged form has one tile: the 128 lanes of tensor memory
@@ -737,8 +738,8 @@ bool ring_info(const KernelRec &k, int *header, int *stage_bytes, int *min_stage
     const int bn = s[9] > 0 ? s[9] : kConvBN;
     const ConvUmmaParams *cp = reinterpret_cast<const ConvUmmaParams *>(k.params);
     const int K = s[1] * s[5] * s[6];
-    if (cp->st.slots) {   // staged: the raw ring stays as registered, the 16 KB weight stages are what can be given up
     if (cp->plane_imgs) return false;   // whole planes: weight and A stages share their barriers, four of each
+    if (cp->st.slots) {   // staged: the raw ring stays as registered, the 16 KB weight stages are what can be given up
       *header = conv_header_bytes(K) + conv_raw_bytes(cp->st.slots, cp->st.slot_pitch), *stage_bytes = kUmmaABytes;
       *min_stages = std::min(2, K / ConvUmmaTf32::kBK);
     } else {
@@ -767,11 +768,11 @@ int launch_fused_rec(bfuse_context *ctx, FusionRec &f, cudaStream_t s, const Dis
   alignas(64) unsigned char pa[kParamsBytes], pb[kParamsBytes];
   DispatchTable with_switch;
   if (ctx->no_pdl) {
-    with_switch = table ? *table : f.plan.table;
+    with_switch = table ? *table : f.launch;
     with_switch.no_pdl = 1;
     table = &with_switch;
   }
-  cudaError_t e = fn(table ? *table : f.plan.table, params_with_stages(a, f.stages[0], pa), params_with_stages(b, f.stages[1], pb), f.launch_grid,
+  cudaError_t e = fn(table ? *table : f.launch, params_with_stages(a, f.stages[0], pa), params_with_stages(b, f.stages[1], pb), f.launch_grid,
                      (unsigned)f.plan.fused_block, f.smem, s);
   if (e != cudaSuccess) return fail_cuda(ctx, e, ("launch " + f.name).c_str());
   return BFUSE_OK;
@@ -1093,12 +1094,44 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
   }
   if (f->smem > kMaxSmemPerCta) return fail(ctx, BFUSE_ERR_SMEM, f->name + ": fused shared memory over the 227 KB per-CTA budget");
   f->launch_grid = (unsigned)f->plan.fused_grid;
+  f->launch = t;
   cudaSetDevice(ctx->device);
   const PairEntry &pe = ctx->pairs[a->desc.op][b->desc.op];
+  const int by_smem = std::max<int>(1, (int)((228 * 1024) / (f->smem + 1024)));   // CTAs an SM's shared memory holds
+  // A memory-bound operator of many small CTAs beside one with tensor memory: every CTA is charged the partner's
+  // shared-memory window, mostly half an SM's, and the SM starts the CTAs of such a kernel one after the other.  Where
+  // at most two fit an SM anyway the pair takes its register-rich build (the other one spills, and its promise of four
+  // CTAs buys nothing), and past two rounds of what is resident the small CTAs take runs of consecutive blocks, two at
+  // a time, so many that both operators together make about two rounds (in one round the partner's slots would idle
+  // once it is done).  Causal QK^T of 6 heads of 1024 tokens beside the softmax of 6 heads (9.6 and 9.1 us alone): 39.0 us,
+  // 27.3 with the register-rich build, 21.2 with runs of 4; PV beside the softmax 31.6, 22.8, 18.2 (runs of 2; 20.0 with 4).
+  // Smaller windows for the GEMM do not help: with four CTAs an SM in 64 registers QK^T || softmax takes 23-28 us.
+  auto memory_bound = [](const KernelRec &k) { return k.desc.op <= BFUSE_OP_ROPE_BF16; };
+  const int row = memory_bound(*a) && tmem_cols(*b) ? 0 : memory_bound(*b) && tmem_cols(*a) ? 1 : -1;
+  const bool row_rich = row >= 0 && by_smem <= pe.wide_min_blocks;
+  if (row_rich && !thread_split && !t.queue) {
+    const int slots = by_smem * ctx->sm_count;
+    const int n_row = kd[row].grid(), n_other = kd[1 - row].grid();
+    const int per = n_row + n_other > 2 * slots ? std::max(2, ceil_div(n_row, std::max(slots, 2 * slots - n_other)) & ~1) : 1;
+    if (per > 1) {
+      KernelDims runs[2] = {kd[0], kd[1]};
+      runs[row].gx = ceil_div(n_row, per);   // (a row-wise operator's grid is one-dimensional)
+      FusedPlan coarse;
+      if (!plan_pair(runs, pattern, param_m, param_n, param_m, &coarse, &err, cluster)) return fail(ctx, BFUSE_ERR_INVALID, err);
+      DispatchTable &l = coarse.table;
+      l.status = t.status;
+      l.smem_off[0] = t.smem_off[0], l.smem_off[1] = t.smem_off[1];
+      l.grid_x[row] = t.grid_x[row];
+      l.per_cta[row] = per;
+      l.n_block[row] = n_row;
+      f->launch = l;
+      f->launch_grid = (unsigned)coarse.fused_grid;
+    }
+  }
   // the register-richer build of the pair when its occupancy still holds the whole grid in one wave
   // (or, for two memory-bound bodies, when the grid is many waves long and waves stop mattering)
   f->wide = !thread_split && pe.block_wide && !t.queue &&
-            (f->launch_grid <= (unsigned)(pe.wide_min_blocks * ctx->sm_count) ||
+            (f->launch_grid <= (unsigned)(pe.wide_min_blocks * ctx->sm_count) || row_rich ||
              (pe.wide_min_blocks == 4 && f->launch_grid >= (unsigned)(12 * ctx->sm_count)));
   cudaFuncAttributes attr;
   cudaError_t e = (thread_split ? pe.thread_attr : (f->wide ? pe.block_wide_attr : pe.block_attr))(&attr);
@@ -1115,6 +1148,7 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
     CK(cudaMalloc(&f->queue_ctr, 2 * sizeof(unsigned)));
     CK(cudaMemset(f->queue_ctr, 0, 2 * sizeof(unsigned)));
     t.queue_ctr = f->queue_ctr;
+    f->launch = t;
   }
   undo.keep = true;
   ++ctx->kernels[f->reg1]->users, ++ctx->kernels[f->reg2]->users;
@@ -1451,7 +1485,7 @@ int bfuse_trace_fused(bfuse_context *ctx, int fusion, int *kernel_of, int *vbloc
   CK(cudaMalloc(&d, 3 * sizeof(int) * cnt));
   cudaError_t e = cudaMemset(d, 0xff, 3 * sizeof(int) * cnt);
   if (e == cudaSuccess) {
-    trace_kernel<<<f->launch_grid, 32, 0, ctx->own>>>(t, d, d + cnt, d + 2 * cnt);
+    trace_kernel<<<t.queue ? f->launch_grid : (unsigned)f->plan.fused_grid, 32, 0, ctx->own>>>(t, d, d + cnt, d + 2 * cnt);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own);
@@ -1482,7 +1516,7 @@ int bfuse_debug_fused_timeline(bfuse_context *ctx, const int *fusions, int n, lo
   size_t off = 0;
   for (int i = 0; i < n && e == cudaSuccess && !rc; ++i) {
     FusionRec *f = get_fusion(ctx, fusions[i]);
-    DispatchTable t = f->plan.table;
+    DispatchTable t = f->launch;
     t.cta_times = d + off * 3;
     rc = launch_fused_rec(ctx, *f, ctx->own, &t);
     off += (size_t)slots[i];

@@ -27,6 +27,7 @@ struct TileCtx {
   int persistent;       // 1: more tensor-memory allocations may follow in this CTA (work queue: the next
                         // tile; thread split: the other operator), so the allocation permit must be kept
   unsigned tmem_base;   // tmem_given: the tensor-memory columns the CTA already holds for this operator (a persistent
+  int waited = 0;       // 1: an earlier tile of this CTA has waited for the previous kernel
   int tmem_given;       // CTA of the work queue allocates once for all its tickets); the body neither allocates nor frees
 
   // Programmatic dependent launch: the CTA may have started while the previous kernel on the stream
@@ -36,6 +37,7 @@ struct TileCtx {
   // Only then is the next kernel allowed to start its CTAs: were it allowed earlier, CTAs of several
   // queued launches would pile up on whatever SMs had room first, holding tensor memory and slots.
   __device__ __forceinline__ void dependency_wait() const {
+    if (waited) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
@@ -94,20 +96,33 @@ struct OpMax {
 // shuffles first; rows wider than a warp exchange one partial per warp through slot `slot` of the
 // operator's shared-memory window and meet on the operator's named barrier.  Successive
 // reductions in one tile use different slots, which keeps the barrier count at one per reduction.
-template <class Op>
-__device__ __forceinline__ float row_reduce(float v, const TileCtx &c, int tpr, int slot) {
+// R rows of a thread at once (R <= 4: a slot has 8 words for each) share that barrier.
+template <class Op, int R>
+__device__ __forceinline__ void row_reduce(float (&v)[R], const TileCtx &c, int tpr, int slot) {
   const int width = tpr < 32 ? tpr : 32;
-  for (int off = width >> 1; off > 0; off >>= 1) v = Op::apply(v, __shfl_xor_sync(0xffffffffu, v, off));
+  for (int off = width >> 1; off > 0; off >>= 1)
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = Op::apply(v[i], __shfl_xor_sync(0xffffffffu, v[i], off));
   if (tpr > 32) {
     float *s = reinterpret_cast<float *>(c.smem) + slot * 32;
-    if ((c.tid & 31) == 0) s[c.tid >> 5] = v;
+    if ((c.tid & 31) == 0)
+#pragma unroll
+      for (int i = 0; i < R; ++i) s[8 * i + (c.tid >> 5)] = v[i];
     c.sync();
     const int wpr = tpr >> 5, w0 = (c.tid / tpr) * wpr;
-    float r = s[w0];
-    for (int j = 1; j < wpr; ++j) r = Op::apply(r, s[w0 + j]);
-    v = r;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float r = s[8 * i + w0];
+      for (int j = 1; j < wpr; ++j) r = Op::apply(r, s[8 * i + w0 + j]);
+      v[i] = r;
+    }
   }
-  return v;
+}
+template <class Op>
+__device__ __forceinline__ float row_reduce(float v, const TileCtx &c, int tpr, int slot) {
+  float a[1] = {v};
+  row_reduce<Op, 1>(a, c, tpr, slot);
+  return a[0];
 }
 
 }  // namespace bfuse

@@ -1,0 +1,46 @@
+"""Fused launches in which the CTAs of a row-wise operator beside a tensor-memory operator take runs of blocks."""
+import numpy as np
+import pytest
+
+import bfuse_project_b200 as bf
+from bfuse_project_b200 import workloads as wl
+from test_gpu_b_pairs import run_and_check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rt():
+    r = bf.Runtime(0)
+    yield r
+    r.close()
+
+
+# enough blocks for runs of 2, 4 and more; a last run cut short, a last block of fewer rows, rows wider than a warp
+@pytest.mark.parametrize("row", [
+    lambda rng: wl.softmax("sm", rng, 7001, 512, 0.125),
+    lambda rng: wl.softmax("sm", rng, 6145, 1024, 0.125),
+    lambda rng: wl.softmax("sm", rng, 20000, 128, 1.0),
+    lambda rng: wl.layernorm("ln", rng, 5003, 768, 1e-5, residual=True),
+    lambda rng: wl.rmsnorm("rms", rng, 4501, 2048, 1e-5),
+    lambda rng: wl.rope("rope", rng, 4099, 8, 128, 500000.0),
+])
+@pytest.mark.parametrize("pattern", [(bf.ZIGZAG, 1, 1), (bf.RANGE_SPLIT, 0, 0)])
+def test_runs_equal_one_block_per_cta(rt, row, pattern):
+    rng = np.random.default_rng(11)
+    g = wl.gemm("g", rng, bf.OP_GEMM_TF32, 2, 200, 256, 64, causal=True, w_std=1.0, bn=256, split=1)   # a window of half an SM
+    for a, b in ((row(rng), g), (g, row(rng))):
+        pair = run_and_check(rt, wl.PairSpec("runs", a, b, "tf32", "hbm"), [pattern])
+        f = pair.fusion(*pattern)
+        info = rt.fusion_info(f)
+        assert info["launched_ctas"] < info["GridDim"][0]
+        assert [rt.map_block(f, i)[0] for i in (0, info["GridDim"][0] - 1)] and len(rt.trace_fused(f)[0]) == info["GridDim"][0]
+
+
+def test_runs_of_clusters(rt):
+    """A k-split GEMM: its partner's CTAs are dealt in clusters, a run to each."""
+    rng = np.random.default_rng(12)
+    g = wl.gemm("g", rng, bf.OP_GEMM_TF32, 1, 256, 256, 1024, w_std=0.05, bn=128, split=4)
+    pair = run_and_check(rt, wl.PairSpec("runs", wl.softmax("sm", rng, 7001, 512, 0.125), g, "tf32", "hbm"), [(bf.ZIGZAG, 1, 1), (bf.RANGE_SPLIT, 0, 0)])
+    info = rt.fusion_info(pair.fusion(bf.ZIGZAG, 1, 1))
+    assert info["launched_ctas"] < info["GridDim"][0]

@@ -37,8 +37,8 @@ struct SoftmaxF32 {
   template <int R>
   __device__ __forceinline__ static void run_rows(const Params &p, const TileCtx &c, int end) {
     c.dependency_wait();
-    const int tpr = c.bx, lane = c.tid % tpr, row0 = c.vblock * c.by + c.tid / tpr;
-    const int nvec = p.cols / (4 * tpr);
+    const int tpr = c.bx, tsh = log2_of(tpr), lane = c.tid & (tpr - 1), row0 = c.vblock * c.by + (c.tid >> tsh);
+    const int nvec = p.cols >> (2 + tsh);
     float4 v[R][kRowMaxVec];
     bool live[R];
     // every load of the rows is issued before the first use of any of them: a use between two loads
@@ -118,8 +118,8 @@ struct LayerNormF32 {
 
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
     c.dependency_wait();
-    const int tpr = c.bx, lane = c.tid % tpr, row = c.vblock * c.by + c.tid / tpr;
-    const int nvec = p.cols / (4 * tpr);
+    const int tpr = c.bx, tsh = log2_of(tpr), lane = c.tid & (tpr - 1), row = c.vblock * c.by + (c.tid >> tsh);
+    const int nvec = p.cols >> (2 + tsh);
     const bool live = row < p.rows;
     const float4 *xr = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.cols);
     const float4 *rr = reinterpret_cast<const float4 *>(p.res + (size_t)row * p.cols);
@@ -202,8 +202,8 @@ struct RmsNormBf16 {
 
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
     c.dependency_wait();
-    const int tpr = c.bx, lane = c.tid % tpr, row = c.vblock * c.by + c.tid / tpr;
-    const int nvec = p.cols / (8 * tpr);
+    const int tpr = c.bx, tsh = log2_of(tpr), lane = c.tid & (tpr - 1), row = c.vblock * c.by + (c.tid >> tsh);
+    const int nvec = p.cols >> (3 + tsh);
     const bool live = row < p.rows;
     const uint4 *xr = reinterpret_cast<const uint4 *>(p.x + (size_t)row * p.cols);
     const uint4 *w4 = reinterpret_cast<const uint4 *>(p.w);
@@ -257,7 +257,10 @@ struct RopeBf16 {
     const float *inv_freq;  // [dim / 2]
     uint16_t *y;
     int seq, heads, dim;
+    int heads_per_group;           // heads of a thread: heads / (BlockDim.X / chunks)
+    int inv_bx, inv_chunks;        // 65536 / d + 1: x / d = x * inv >> 16, exact for x, d <= 256
   };
+  __host__ __device__ static constexpr int inverse(int d) { return 65536 / d + 1; }
   static constexpr int kMaxThreads = 256;
   static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40 (32 spills badly; 5 CTAs of 48 registers lose more in waves than the spills cost)
   static constexpr bool kMemoryBound = true;
@@ -266,8 +269,8 @@ struct RopeBf16 {
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
     c.dependency_wait();
     const int half = p.dim >> 1, chunks = half >> 3;
-    const int tx = c.tid % c.bx, chunk = tx % chunks, hg = tx / chunks, ngroups = c.bx / chunks;
-    const int pos = c.vblock * c.by + c.tid / c.bx;
+    const int ty = c.tid * p.inv_bx >> 16, tx = c.tid - ty * c.bx, hg = tx * p.inv_chunks >> 16, chunk = tx - hg * chunks;
+    const int pos = c.vblock * c.by + ty;
     if (pos >= p.seq) return;
     // The frequency table first (the sin / cos arithmetic waits for it), then all of this thread's
     // rows as L1 prefetches that tie up no register; the arithmetic runs while they travel and the
@@ -275,7 +278,7 @@ struct RopeBf16 {
     // queue behind everything the grid already has in flight and cost another trip to DRAM per head.
     const float4 f0 = __ldg(reinterpret_cast<const float4 *>(p.inv_freq) + chunk * 2);
     const float4 f1 = __ldg(reinterpret_cast<const float4 *>(p.inv_freq) + chunk * 2 + 1);
-    const int hpt = p.heads / ngroups, h_begin = hg * hpt, h_end = h_begin + hpt;
+    const int hpt = p.heads_per_group, h_begin = hg * hpt, h_end = h_begin + hpt;
     const size_t o0 = ((size_t)pos * p.heads + h_begin) * p.dim + chunk * 8;
     for (int h = 0; h < hpt; ++h) {
       prefetch_l1(p.q + o0 + (size_t)h * p.dim);

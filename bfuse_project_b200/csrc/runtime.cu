@@ -481,7 +481,8 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
       const int chunks = s[2] / 16;
       if (kd.bx % chunks || s[1] % (kd.bx / chunks) || kd.bz != 1) return shape_err("BlockDim.X must be chunks * (a divisor of heads)");
       if (kd.gy != 1 || kd.gz != 1 || (long long)kd.gx * kd.by < s[0]) return shape_err("GridDim.X * positions per CTA must cover seq");
-      RopeBf16::Params p{(const uint16_t *)a[0], (const float *)a[1], (uint16_t *)a[2], s[0], s[1], s[2]};
+      RopeBf16::Params p{(const uint16_t *)a[0], (const float *)a[1], (uint16_t *)a[2], s[0], s[1], s[2],
+                         s[1] / (kd.bx / chunks), RopeBf16::inverse(kd.bx), RopeBf16::inverse(chunks)};
       std::memcpy(k.params, &p, sizeof(p));
       return BFUSE_OK;
     }

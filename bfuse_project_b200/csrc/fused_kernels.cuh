@@ -5,8 +5,8 @@
 // pair of operator bodies from the registry:
 //
 //   fused_block_kernel<A, B>   every CTA runs one operator (zig-zag, proportional, SM-striped,
-//                              range split) or, with table.queue set, loops over tickets drawn
-//                              from an atomic counter (persistent work queue);
+//                              range split);
+//   fused_queue_kernel<A, B>   persistent CTAs loop over tickets drawn from an atomic counter (work queue);
 //   fused_thread_kernel<A, B>  both operators inside every CTA, split by thread range, each
 //                              synchronising on its own named barrier; shared memory is the sum;
 //   fused_group_kernel<A>      up to four operators of one body in one launch (the reference's
@@ -78,7 +78,7 @@ __device__ __forceinline__ void run_tile(const typename Op::Params &p, const Dis
 // bfuse_register_fusion for when CTAs take runs.
 template <class Op, bool RUNS>
 __device__ __forceinline__ void run_blocks(const typename Op::Params &p, const DispatchTable &t, int k, int vb, int vtid,
-                                           int bar_id, unsigned char *smem, int tmem_given, unsigned tmem_base) {
+                                           int bar_id, unsigned char *smem) {
   if constexpr (RUNS) {
     if (t.per_cta[k] > 1) {
       const int end = min((vb + 1) * t.per_cta[k], t.n_block[k]);
@@ -94,7 +94,7 @@ __device__ __forceinline__ void run_blocks(const typename Op::Params &p, const D
       return;
     }
   }
-  run_tile<Op>(p, t, k, vb, vtid, bar_id, smem, 0, tmem_given, tmem_base);
+  run_tile<Op>(p, t, k, vb, vtid, bar_id, smem);
 }
 
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
@@ -110,15 +110,19 @@ constexpr int pair_min_blocks() {
 
 // A second, register-richer build of pairs with a memory-bound body, launched when its occupancy
 // still holds the whole fused grid (so nothing is lost in waves).  Two memory-bound bodies: 4 CTAs
-// per SM (64 registers) -- under the 40-register cap of the 6-CTA build the two inlined bodies spill.
-// A memory-bound body beside a GEMM / conv body: 2 CTAs per SM (128 registers) -- the 64 registers
-// of the default build make the tensor-core body's epilogue spill.  0: the pair has no second build.
+// per SM (64 registers), which let a thread keep more loads in flight than the 40 of the 6-CTA build.
+// A memory-bound body beside a GEMM / conv body: 2 CTAs per SM (128 registers), for the tensor-core
+// body's epilogue and for rows taken two at a time (run_blocks).  0: the pair has no second build.
 template <class A, class B>
 constexpr int pair_wide_blocks() {
   return (A::kMemoryBound && B::kMemoryBound) ? (pair_min_blocks<A, B>() > 4 ? 4 : 0)
                                               : ((A::kMemoryBound || B::kMemoryBound) && pair_min_blocks<A, B>() > 2 ? 2 : 0);
 }
 
+// One CTA, one dispatch slot.  The persistent form is a kernel of its own (fused_queue_kernel): with both in one loop
+// the state that loop carries made every pair with a memory-bound body spill (softmax || LayerNorm 324 bytes a thread in
+// the 40-register build and 44 in the 64-register one, 4 and none without it: 12 launches at 512 tokens 79.3 -> 67.7 us,
+// one at 6007 tokens 64.0 -> 51.4).
 template <class A, class B, int MINB = pair_min_blocks<A, B>()>
 __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
     fused_block_kernel(const __grid_constant__ DispatchTable t, const __grid_constant__ typename A::Params pa,
@@ -128,24 +132,49 @@ __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
   const int tid = threadIdx.x;
   unsigned long long t_entry = 0;
   if (t.cta_times) t_entry = global_timer_ns();
+  int k = 0, vb = 0;
+  const bool mapped = decode_cta(t, blockIdx.x, k, vb);
   // A kernel that contains tcgen05.alloc gets its CTAs launched one at a time per SM: the next CTA
   // starts only once the resident one has given up its permit to allocate tensor memory, and a CTA
   // that never allocates holds it until it exits.  So the CTAs of an operator without tensor memory
   // give the permit up before anything else (measured: 4 such CTAs per SM ran one after the other).
   if constexpr (A::kUsesTmem != B::kUsesTmem) {
-    if (!t.queue && tid < 32) {
-      int k0, vb0;
-      const bool mapped = decode_cta(t, blockIdx.x, k0, vb0);
-      if (!mapped || (k0 == 0 ? !A::kUsesTmem : !B::kUsesTmem)) relinquish_tmem_permit();
-    }
+    if (tid < 32 && (!mapped || (k == 0 ? !A::kUsesTmem : !B::kUsesTmem))) relinquish_tmem_permit();
   }
-  // A persistent CTA of the work queue allocates the tensor memory its operators need ONCE, for all its
+  if (!mapped) return;
+  // kernel entry, body start (its set-up may overlap the previous kernel), thread 0 done: each mark goes out as it is
+  // taken -- the buffer is the launch's own -- for held to the end they would cost the bodies registers
+  if (t.cta_times && tid == 0) {
+    t.cta_times[3 * (size_t)blockIdx.x] = t_entry;
+    t.cta_times[3 * (size_t)blockIdx.x + 1] = global_timer_ns();
+  }
+  // guard of the reference: KernelID_ == k && threadIdx.x < B_k (Algorithms.cc:699-717)
+  if (k == 0) {
+    if (tid < t.n_thr[0]) run_blocks<A, A::kMemoryBound && B::kUsesTmem && MINB == 2>(pa, t, 0, vb, tid, 1, smem);
+  } else {
+    if (tid < t.n_thr[1]) run_blocks<B, B::kMemoryBound && A::kUsesTmem && MINB == 2>(pb, t, 1, vb, tid, 2, smem);
+  }
+  if (t.cta_times && tid == 0) t.cta_times[3 * (size_t)blockIdx.x + 2] = global_timer_ns();
+}
+
+// Persistent CTAs that draw tickets from an atomic counter until the queue is empty.  The last CTA to drain
+// resets the counters, so the next launch on the stream starts from zero without a memset.
+template <class A, class B>
+__global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), (pair_min_blocks<A, B>()))
+    fused_queue_kernel(const __grid_constant__ DispatchTable t, const __grid_constant__ typename A::Params pa,
+                       const __grid_constant__ typename B::Params pb) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *smem = align_smem_1k(smem_raw);
+  const int tid = threadIdx.x;
+  unsigned long long t_entry = 0;
+  if (t.cta_times) t_entry = global_timer_ns();
+  // A persistent CTA allocates the tensor memory its operators need ONCE, for all its
   // tickets, and gives the permit up at once: the SM starts the next CTA of a tcgen05 kernel only when the
   // resident one has given the permit up, so a persistent CTA that kept it for a later ticket held the SM's
   // second CTA off for the whole launch (batch-256 conv pair: 281 us, against 161 us for a plain launch).
   __shared__ unsigned queue_tmem_s;
   unsigned queue_tmem = 0;
-  const int queue_tmem_cols = (A::kUsesTmem || B::kUsesTmem) && t.queue ? t.tmem_cols : 0;
+  const int queue_tmem_cols = A::kUsesTmem || B::kUsesTmem ? t.tmem_cols : 0;
   if (queue_tmem_cols > 0) {
     if (tid < 32) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(&queue_tmem_s)),
@@ -158,38 +187,27 @@ __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     queue_tmem = *reinterpret_cast<volatile unsigned *>(&queue_tmem_s);
   }
-  if (t.queue) {   // the ticket counter is global memory; otherwise the body waits and lets the next kernel in (TileCtx::dependency_wait)
-    grid_dependency_wait();
-    // A queue launch with a tensor-memory operator does not let the next kernel in early: CTAs of a
-    // following tensor-memory kernel, started early, allocate their columns before their own
-    // griddepcontrol.wait and would hold them on this SM until this grid has finished, beside persistent
-    // CTAs that are here for the whole launch.  Two memory-bound bodies keep the early trigger.
-    if constexpr (!A::kUsesTmem && !B::kUsesTmem) grid_launch_dependents();
-  }
-  // One loop serves both launch forms, so each body is inlined once (two copies cost registers and
-  // made the memory-bound pairs spill): a plain launch runs it for CTA blockIdx.x and leaves; a
-  // persistent CTA of the work queue draws tickets until the queue is empty.  The last CTA to drain
-  // resets the counters, so the next launch on the stream starts from zero without a memset.
+  grid_dependency_wait();   // the ticket counter is global memory
+  // A queue launch with a tensor-memory operator does not let the next kernel in early: CTAs of a
+  // following tensor-memory kernel, started early, allocate their columns before their own
+  // griddepcontrol.wait and would hold them on this SM until this grid has finished, beside persistent
+  // CTAs that are here for the whole launch.  Two memory-bound bodies keep the early trigger.
+  if constexpr (!A::kUsesTmem && !B::kUsesTmem) grid_launch_dependents();
   __shared__ int ticket_s;
-  const bool queue = t.queue != 0;
-  int ticket = blockIdx.x;
-  do {
-    if (queue) {
-      if (tid == 0) ticket_s = (int)atomicAdd(t.queue_ctr, 1u);
-      __syncthreads();
-      ticket = ticket_s;
-      __syncthreads();
-      if (ticket >= t.total) break;
-    }
+  for (;;) {
+    if (tid == 0) ticket_s = (int)atomicAdd(t.queue_ctr, 1u);
+    __syncthreads();
+    const int ticket = ticket_s;
+    __syncthreads();
+    if (ticket >= t.total) break;
     int k, vb;
     if (decode_cta(t, ticket, k, vb)) {
       unsigned long long t_body = 0;
       if (t.cta_times) t_body = global_timer_ns();
-      // guard of the reference: KernelID_ == k && threadIdx.x < B_k (Algorithms.cc:699-717)
       if (k == 0) {
-        if (tid < t.n_thr[0]) run_blocks<A, A::kMemoryBound && B::kUsesTmem && MINB == 2>(pa, t, 0, vb, tid, 1, smem, queue_tmem_cols > 0, queue_tmem);
+        if (tid < t.n_thr[0]) run_tile<A>(pa, t, 0, vb, tid, 1, smem, 0, queue_tmem_cols > 0, queue_tmem);
       } else {
-        if (tid < t.n_thr[1]) run_blocks<B, B::kMemoryBound && A::kUsesTmem && MINB == 2>(pb, t, 1, vb, tid, 2, smem, queue_tmem_cols > 0, queue_tmem);
+        if (tid < t.n_thr[1]) run_tile<B>(pb, t, 1, vb, tid, 2, smem, 0, queue_tmem_cols > 0, queue_tmem);
       }
       if (t.cta_times && tid == 0) {  // kernel entry, body start (its set-up may overlap the previous kernel), thread 0 done
         t.cta_times[3 * (size_t)ticket] = t_entry;
@@ -197,13 +215,13 @@ __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
         t.cta_times[3 * (size_t)ticket + 2] = global_timer_ns();
       }
     }
-  } while (queue);
+  }
   if (queue_tmem_cols > 0) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tid < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(queue_tmem), "r"(queue_tmem_cols) : "memory");
   }
-  if (queue && tid == 0) {
+  if (tid == 0) {
     __threadfence();
     if (atomicAdd(t.queue_ctr + 1, 1u) == gridDim.x - 1) {
       t.queue_ctr[0] = 0;
@@ -401,6 +419,14 @@ cudaError_t launch_block_pair(const DispatchTable &t, const void *pa, const void
                           *static_cast<const typename A::Params *>(pa), *static_cast<const typename B::Params *>(pb));
 }
 template <class A, class B>
+cudaError_t launch_queue_pair(const DispatchTable &t, const void *pa, const void *pb, unsigned grid, unsigned block,
+                              size_t smem, cudaStream_t s) {
+  cudaError_t e = ensure_smem(fused_queue_kernel<A, B>, smem);
+  if (e != cudaSuccess) return e;
+  return launch_clustered(fused_queue_kernel<A, B>, grid, block, smem, s, 1, !t.no_pdl, t,
+                          *static_cast<const typename A::Params *>(pa), *static_cast<const typename B::Params *>(pb));
+}
+template <class A, class B>
 cudaError_t launch_thread_pair(const DispatchTable &t, const void *pa, const void *pb, unsigned grid, unsigned block,
                                size_t smem, cudaStream_t s) {
   cudaError_t e = ensure_smem(fused_thread_kernel<A, B>, smem);
@@ -460,6 +486,8 @@ cudaError_t attr_block_pair_wide(cudaFuncAttributes *a) {
 }
 template <class A, class B>
 cudaError_t attr_block_pair(cudaFuncAttributes *a) { return cudaFuncGetAttributes(a, fused_block_kernel<A, B>); }
+template <class A, class B>
+cudaError_t attr_queue_pair(cudaFuncAttributes *a) { return cudaFuncGetAttributes(a, fused_queue_kernel<A, B>); }
 template <class A, class B>
 cudaError_t attr_thread_pair(cudaFuncAttributes *a) { return cudaFuncGetAttributes(a, fused_thread_kernel<A, B>); }
 template <class A>

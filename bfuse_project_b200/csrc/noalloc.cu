@@ -80,7 +80,7 @@ extern "C" int bfuse_softmax_layernorm_queue_noalloc(const float *sm_x, float *s
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices) return reject(BFUSE_ERR_DEVICE, "no current CUDA device");
   DeviceSetup &su = g_setup[dev];
-  auto kernel = fused_block_kernel<SoftmaxF32, LayerNormF32>;
+  auto kernel = fused_queue_kernel<SoftmaxF32, LayerNormF32>;
   std::call_once(su.once, [&] {
     // once per device, with that device current: the array's name is a host-side handle, the
     // kernel needs its device address

@@ -27,7 +27,7 @@ struct SoftmaxF32 {
     float scale;
   };
   static constexpr int kMaxThreads = 256;
-  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40 (32 spills badly; 5 CTAs of 48 registers lose more in waves than the spills cost)
+  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40
   static constexpr bool kMemoryBound = true;
   static constexpr bool kUsesTmem = false;   // allocates tensor memory (see fused_block_kernel)
 
@@ -36,9 +36,11 @@ struct SoftmaxF32 {
   // R consecutive virtual blocks at once, c.vblock first and none at or past `end`: a thread has a row of each.
   template <int R>
   __device__ __forceinline__ static void run_rows(const Params &p, const TileCtx &c, int end) {
-    c.dependency_wait();
     const int tpr = c.bx, tsh = log2_of(tpr), lane = c.tid & (tpr - 1), row0 = c.vblock * c.by + (c.tid >> tsh);
     const int nvec = p.cols >> (2 + tsh);
+    if (c.may_start_early() && (lane & 7) == 0 && row0 < p.rows)
+      for (int i = 0; i < nvec; ++i) prefetch_l2(p.x + (size_t)row0 * p.cols + 4 * (i * tpr + lane));
+    c.dependency_wait();
     float4 v[R][kRowMaxVec];
     bool live[R];
     // every load of the rows is issued before the first use of any of them: a use between two loads
@@ -112,14 +114,16 @@ struct LayerNormF32 {
     float eps;
   };
   static constexpr int kMaxThreads = 256;
-  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40 (32 spills badly; 5 CTAs of 48 registers lose more in waves than the spills cost)
+  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40
   static constexpr bool kMemoryBound = true;
   static constexpr bool kUsesTmem = false;   // allocates tensor memory (see fused_block_kernel)
 
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
-    c.dependency_wait();
     const int tpr = c.bx, tsh = log2_of(tpr), lane = c.tid & (tpr - 1), row = c.vblock * c.by + (c.tid >> tsh);
     const int nvec = p.cols >> (2 + tsh);
+    if (c.may_start_early() && (lane & 7) == 0 && row < p.rows)
+      for (int i = 0; i < nvec; ++i) prefetch_l2(p.x + (size_t)row * p.cols + 4 * (i * tpr + lane));
+    c.dependency_wait();
     const bool live = row < p.rows;
     const float4 *xr = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.cols);
     const float4 *rr = reinterpret_cast<const float4 *>(p.res + (size_t)row * p.cols);
@@ -195,15 +199,15 @@ struct RmsNormBf16 {
     float eps;
   };
   static constexpr int kMaxThreads = 256;
-  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40 (32 spills badly; 5 CTAs of 48 registers lose more in waves than the spills cost)
+  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40
   static constexpr bool kMemoryBound = true;
   static constexpr bool kUsesTmem = false;   // allocates tensor memory (see fused_block_kernel)
   static constexpr int kMaxVec = 4;  // 8 bf16 per vector
 
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
-    c.dependency_wait();
     const int tpr = c.bx, tsh = log2_of(tpr), lane = c.tid & (tpr - 1), row = c.vblock * c.by + (c.tid >> tsh);
     const int nvec = p.cols >> (3 + tsh);
+    c.dependency_wait();
     const bool live = row < p.rows;
     const uint4 *xr = reinterpret_cast<const uint4 *>(p.x + (size_t)row * p.cols);
     const uint4 *w4 = reinterpret_cast<const uint4 *>(p.w);
@@ -262,15 +266,15 @@ struct RopeBf16 {
   };
   __host__ __device__ static constexpr int inverse(int d) { return 65536 / d + 1; }
   static constexpr int kMaxThreads = 256;
-  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40 (32 spills badly; 5 CTAs of 48 registers lose more in waves than the spills cost)
+  static constexpr int kMinBlocks = 6;   // 6 x 256 threads per SM: registers per thread <= 40
   static constexpr bool kMemoryBound = true;
   static constexpr bool kUsesTmem = false;   // allocates tensor memory (see fused_block_kernel)
 
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
-    c.dependency_wait();
     const int half = p.dim >> 1, chunks = half >> 3;
     const int ty = c.tid * p.inv_bx >> 16, tx = c.tid - ty * c.bx, hg = tx * p.inv_chunks >> 16, chunk = tx - hg * chunks;
     const int pos = c.vblock * c.by + ty;
+    c.dependency_wait();
     if (pos >= p.seq) return;
     // The frequency table first (the sin / cos arithmetic waits for it), then all of this thread's
     // rows as L1 prefetches that tie up no register; the arithmetic runs while they travel and the

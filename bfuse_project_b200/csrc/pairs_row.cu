@@ -48,8 +48,10 @@ struct RowFiller {
     using B = typename OpAt<J>::type;
     row[J].block = &launch_block_pair<A, B>;
     row[J].thread = &launch_thread_pair<A, B>;
+    row[J].queue = &launch_queue_pair<A, B>;
     row[J].block_attr = &attr_block_pair<A, B>;
     row[J].thread_attr = &attr_thread_pair<A, B>;
+    row[J].queue_attr = &attr_queue_pair<A, B>;
     row[J].block_clusters = &clusters_block_pair<A, B>;
     WideFiller<A, B, (pair_wide_blocks<A, B>() > 0)>::fill(row[J]);
     MixedFiller<A, B, (I < J)>::fill(row[J]);

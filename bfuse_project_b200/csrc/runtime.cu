@@ -765,7 +765,7 @@ const void *params_with_stages(const KernelRec &k, int stages, unsigned char *sc
 int launch_fused_rec(bfuse_context *ctx, FusionRec &f, cudaStream_t s, const DispatchTable *table = nullptr) {
   KernelRec &a = *ctx->kernels[f.k1], &b = *ctx->kernels[f.k2];
   const PairEntry &pe = ctx->pairs[a.desc.op][b.desc.op];
-  PairLaunchFn fn = f.plan.table.kind == DISPATCH_THREADS ? pe.thread : (f.wide ? pe.block_wide : pe.block);
+  PairLaunchFn fn = f.plan.table.kind == DISPATCH_THREADS ? pe.thread : f.plan.table.queue ? pe.queue : (f.wide ? pe.block_wide : pe.block);
   alignas(64) unsigned char pa[kParamsBytes], pb[kParamsBytes];
   DispatchTable with_switch;
   if (ctx->no_pdl) {
@@ -1129,13 +1129,13 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
       f->launch_grid = (unsigned)coarse.fused_grid;
     }
   }
-  // the register-richer build of the pair when its occupancy still holds the whole grid in one wave
-  // (or, for two memory-bound bodies, when the grid is many waves long and waves stop mattering)
+  // the register-richer build of the pair when its occupancy still holds the whole grid in one wave (of two
+  // memory-bound bodies: RMSNorm || RoPE of 1500 tokens, 16 heads of 64, alone 3.6 us against 4.5 with six CTAs an SM;
+  // longer grids want the six: softmax || LayerNorm of 6007 tokens 51.4 us against 56.4)
   f->wide = !thread_split && pe.block_wide && !t.queue &&
-            (f->launch_grid <= (unsigned)(pe.wide_min_blocks * ctx->sm_count) || row_rich ||
-             (pe.wide_min_blocks == 4 && f->launch_grid >= (unsigned)(12 * ctx->sm_count)));
+            (f->launch_grid <= (unsigned)(pe.wide_min_blocks * ctx->sm_count) || row_rich);
   cudaFuncAttributes attr;
-  cudaError_t e = (thread_split ? pe.thread_attr : (f->wide ? pe.block_wide_attr : pe.block_attr))(&attr);
+  cudaError_t e = (thread_split ? pe.thread_attr : t.queue ? pe.queue_attr : (f->wide ? pe.block_wide_attr : pe.block_attr))(&attr);
   if (e != cudaSuccess) return fail_cuda(ctx, e, "cudaFuncGetAttributes");
   f->regs = attr.numRegs;
   if (t.queue) {

@@ -42,6 +42,11 @@ struct TileCtx {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
 
+  // Is this CTA among those that mostly start under the previous kernel's tail?  Three a SM, of a grid that is not
+  // many rounds long (softmax || LayerNorm of 512 tokens, 12 launches in a row: two a SM 81.3 us, three 79.3, four 80.0,
+  // all 84.0, none 92.8: a CTA that finds the wait over pays for its prefetches and gains nothing).
+  __device__ __forceinline__ bool may_start_early() const { return !waited && !persistent && blockIdx.x < 148 * 3 && gridDim.x <= 148 * 12; }
+
   __device__ __forceinline__ void sync() const {
     asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(bar_count) : "memory");
   }
@@ -89,6 +94,10 @@ __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefe
 // costs a CTA a hundred clocks and more before its first load leaves (three to six of them in the row-wise bodies:
 // a lone softmax || LayerNorm of 64 tokens 3.68 -> 3.42 us, RMSNorm || RoPE of 512 tokens 6.6 -> 6.1 us a layer)
 __device__ __forceinline__ int log2_of(int x) { return 31 - __clz(x); }
+
+// Ask for the line at p to be brought into L2.  A hint without a value: it may go out before dependency_wait(), while
+// the previous kernel -- which may even be writing there -- still runs, and moves the trip to DRAM under its tail.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 struct OpSum {
   __device__ __forceinline__ static float apply(float a, float b) { return a + b; }

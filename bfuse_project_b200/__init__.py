@@ -309,7 +309,7 @@ class Runtime:
         self._ck(self._L.bfuse_fusion_info(self._ctx, fusion, d))
         return {"KernelName": d.KernelName.decode(), "GridDim": d.GridDim.tuple(), "BlockDim": d.BlockDim.tuple(),
                 "Reg": d.Reg, "smem_bytes": d.smem_bytes, "launched_ctas": d.shape[0], "resident_ctas": d.shape[1],
-                "retiled_unsplit": (bool(d.shape[2]), bool(d.shape[3]))}
+                "retiled_unsplit": (bool(d.shape[2]), bool(d.shape[3])), "blocks_per_cta": (d.shape[4], d.shape[5])}
 
     def map_block(self, fusion, b):
         k, vb = C.c_int(), C.c_int()

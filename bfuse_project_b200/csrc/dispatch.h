@@ -110,6 +110,28 @@ BFUSE_HD bool decode_cta(const DispatchTable &t, int b, int &k, int &vb) {
   return vb < t.n_cta[k];
 }
 
+// The dispatch slots of launched CTA b: operator k, first virtual block vb, first slot and how many.  A slot is one
+// virtual block, numbered in the order of the CTAs that run them: with one block a CTA (no per_cta) the slot is the CTA,
+// and a CTA that takes a run of blocks has as many consecutive slots as its run has blocks.  Every pattern hands out an
+// operator's units in ascending order, so before a CTA of operator k come the blocks of its own lower units and those of
+// the units left over, the other operator's.  Returns false for an unmapped or padding CTA.
+BFUSE_HD bool cta_slots(const DispatchTable &t, int b, int &k, int &vb, int &first, int &count) {
+  if (!decode_cta(t, b, k, vb)) return false;
+  first = b, count = 1;
+  if (t.per_cta[0] <= 1 && t.per_cta[1] <= 1) return true;
+  const int cl = t.cluster > 1 ? t.cluster : 1, other = 1 - k, run = vb;
+  int before = (b / cl - run / cl) * cl;   // CTAs of the other operator (its last cluster may be partly filled)
+  if (before > t.n_cta[other]) before = t.n_cta[other];
+  for (int i = 0; i < 2; ++i) {
+    const int op = i == 0 ? k : other, n = i == 0 ? run : before, per = t.per_cta[op];
+    const int blocks = per > 1 ? (n * per < t.n_block[op] ? n * per : t.n_block[op]) : n;
+    if (i == 0) vb = first = blocks;
+    else first += blocks;
+  }
+  if (t.per_cta[k] > 1) count = t.n_block[k] - vb < t.per_cta[k] ? t.n_block[k] - vb : t.per_cta[k];
+  return true;
+}
+
 // ---- n operators of one body in one launch ------------------------------------------------------
 // The reference writes its patterns for n kernels (Algorithms.cc:323-375, 538-587) although its
 // test suite only ever fuses two.  A group is that general form for up to kGroupMax operators that

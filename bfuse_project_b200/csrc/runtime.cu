@@ -643,12 +643,16 @@ __global__ void trace_kernel(const __grid_constant__ DispatchTable t, int *kerne
   unsigned smid;
   asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
   if (!t.queue) {
-    int k = -1, vb = -1;
-    decode_cta(t, blockIdx.x, k, vb);
-    if (threadIdx.x == 0) {
-      kernel_of[blockIdx.x] = k;
-      vblock_of[blockIdx.x] = vb;
-      sm_of[blockIdx.x] = (int)smid;
+    int k = -1, vb = -1, first = blockIdx.x, count = 1;
+    const bool runs = t.per_cta[0] > 1 || t.per_cta[1] > 1;
+    if (!cta_slots(t, blockIdx.x, k, vb, first, count)) {
+      if (runs) return;   // padding CTAs have a slot only where slots are CTAs
+      k = vb = -1;
+    }
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+      kernel_of[first + i] = k;
+      vblock_of[first + i] = vb + i;
+      sm_of[first + i] = (int)smid;
     }
     return;
   }
@@ -699,6 +703,9 @@ int free_slot(std::vector<std::unique_ptr<T>> &v) {
 FusionRec *get_fusion(const bfuse_context *ctx, int h) {
   return (ctx && h >= 0 && h < (int)ctx->fusions.size()) ? ctx->fusions[h].get() : nullptr;
 }
+
+// Do CTAs of this fusion's launch take runs of virtual blocks (fewer CTAs than dispatch slots)?
+bool takes_runs(const FusionRec &f) { return f.launch.per_cta[0] > 1 || f.launch.per_cta[1] > 1; }
 
 DispatchTable single_table(const bfuse_context *ctx, const KernelRec &k) {
   DispatchTable t;
@@ -1318,13 +1325,14 @@ int bfuse_fusion_info(bfuse_context *ctx, int fusion, bfuse_kernel_desc *out) {
   out->ExecTime = -1.f;
   out->op = -1;
   out->smem_bytes = f->smem;
-  out->shape[0] = (int)f->launch_grid;  // CTAs actually launched (differs from GridDim for the work queue)
+  out->shape[0] = (int)f->launch_grid;  // CTAs actually launched (fewer than GridDim for the work queue and for runs of blocks)
   // CTAs of this kernel resident at once according to the occupancy calculator (whole clusters; one CTA per SM
   // for kernels that allocate tensor memory), 0 when not asked
   out->shape[1] = 0;
   // operator 1 / 2 runs here in a one-k-slice re-tiling of the registered kernel (thread split, work queue)
   out->shape[2] = f->retiled[0] ? 1 : 0;
   out->shape[3] = f->retiled[1] ? 1 : 0;
+  for (int i = 0; i < 2; ++i) out->shape[4 + i] = std::max(1, f->launch.per_cta[i]);   // virtual blocks a launched CTA takes
   if (f->plan.table.kind != DISPATCH_THREADS && !f->wide) {
     const int cl = std::max(1, f->plan.table.cluster);
     cudaSetDevice(ctx->device);
@@ -1338,6 +1346,20 @@ int bfuse_fusion_map_block(const bfuse_context *ctx, int fusion, int b, int *ker
   FusionRec *f = get_fusion(ctx, fusion);
   if (!f || !kernel || !vblock || b < 0) return BFUSE_ERR_INVALID;
   int k, vb;
+  if (takes_runs(*f)) {
+    // the last launched CTA whose first slot is at or below b (padding CTAs have no slots and are stepped over)
+    int lo = 0, hi = (int)f->launch_grid, first = 0, count = 0;
+    while (hi - lo > 1) {
+      const int mid = lo + (hi - lo) / 2;
+      int at = mid;
+      while (at < hi && !cta_slots(f->launch, at, k, vb, first, count)) ++at;
+      if (at == hi || first > b) hi = mid;
+      else lo = at;
+    }
+    if (!cta_slots(f->launch, lo, k, vb, first, count) || b >= first + count) return BFUSE_ERR_INVALID;
+    *kernel = k, *vblock = vb + (b - first);
+    return BFUSE_OK;
+  }
   const int limit = f->plan.table.queue ? f->plan.table.total : f->plan.fused_grid;
   if (b >= limit || !decode_cta(f->plan.table, b, k, vb)) return BFUSE_ERR_INVALID;
   *kernel = k, *vblock = vb;
@@ -1477,7 +1499,7 @@ int bfuse_graph_launch(bfuse_context *ctx, int graph, void *stream) {
 int bfuse_trace_fused(bfuse_context *ctx, int fusion, int *kernel_of, int *vblock_of, int *sm_of, int n) {
   FusionRec *f = get_fusion(ctx, fusion);
   if (!f || !kernel_of || !vblock_of || !sm_of) return fail(ctx, BFUSE_ERR_INVALID, "bad fusion handle");
-  const DispatchTable &t = f->plan.table;
+  const DispatchTable &t = f->launch;
   if (t.kind == DISPATCH_THREADS) return fail(ctx, BFUSE_ERR_UNSUPPORTED, "thread-split fusions host both operators in every CTA");
   const int cnt = t.queue ? t.total : f->plan.fused_grid;
   if (n < cnt) return fail(ctx, BFUSE_ERR_INVALID, "trace arrays shorter than the fused grid");
@@ -1486,7 +1508,7 @@ int bfuse_trace_fused(bfuse_context *ctx, int fusion, int *kernel_of, int *vbloc
   CK(cudaMalloc(&d, 3 * sizeof(int) * cnt));
   cudaError_t e = cudaMemset(d, 0xff, 3 * sizeof(int) * cnt);
   if (e == cudaSuccess) {
-    trace_kernel<<<t.queue ? f->launch_grid : (unsigned)f->plan.fused_grid, 32, 0, ctx->own>>>(t, d, d + cnt, d + 2 * cnt);
+    trace_kernel<<<f->launch_grid, 32, 0, ctx->own>>>(t, d, d + cnt, d + 2 * cnt);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->own);
@@ -1505,7 +1527,7 @@ int bfuse_debug_fused_timeline(bfuse_context *ctx, const int *fusions, int n, lo
     FusionRec *f = get_fusion(ctx, fusions[i]);
     if (!f) return fail(ctx, BFUSE_ERR_INVALID, "bad fusion handle in list");
     if (f->plan.table.kind == DISPATCH_THREADS) return fail(ctx, BFUSE_ERR_UNSUPPORTED, "thread-level fusions record no per-CTA times");
-    const int cnt = f->plan.table.queue ? f->plan.table.total * f->plan.table.cluster : (int)f->launch_grid;
+    const int cnt = f->plan.table.queue ? f->plan.table.total * f->plan.table.cluster : f->plan.fused_grid;
     if (slots[i] < cnt) return fail(ctx, BFUSE_ERR_INVALID, "times array shorter than the fused grid");
     total += (size_t)slots[i];
   }
@@ -1527,6 +1549,21 @@ int bfuse_debug_fused_timeline(bfuse_context *ctx, const int *fusions, int n, lo
   cudaFree(d);
   if (rc) return rc;
   if (e != cudaSuccess) return fail_cuda(ctx, e, "fused timeline");
+  // the kernel records by launched CTA; a CTA that took a run of blocks gives its marks to each of its slots
+  off = 0;
+  for (int i = 0; i < n; ++i) {
+    const FusionRec *f = get_fusion(ctx, fusions[i]);
+    long long *t = times + off * 3;
+    if (takes_runs(*f)) {
+      const std::vector<long long> by_cta(t, t + 3 * (size_t)f->launch_grid);
+      std::fill(t, t + 3 * (size_t)slots[i], 0LL);
+      int k, vb, first, count;
+      for (int b = 0; b < (int)f->launch_grid; ++b)
+        if (cta_slots(f->launch, b, k, vb, first, count))
+          for (int s = first; s < first + count; ++s) std::copy(&by_cta[3 * (size_t)b], &by_cta[3 * (size_t)b] + 3, t + 3 * (size_t)s);
+    }
+    off += (size_t)slots[i];
+  }
   return BFUSE_OK;
 }
 

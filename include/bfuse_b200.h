@@ -137,7 +137,9 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
                           int *fusion);
 /* The record fuse::bfuse / hfuse write to {b,h}fuse_kernels.yaml (src/Fuse.cc:203-220,358-375):
  * name "<k1>_<k2>_fused_{bfuse,hfuse}", fused GridDim / BlockDim, plus smem and registers;
- * shape[0] = CTAs launched, shape[1] = CTAs of the kernel resident at once according to cudaOccupancyMaxActiveClusters,
+ * GridDim counts the pattern's dispatch slots, one virtual block each; shape[0] = CTAs launched, fewer where persistent CTAs
+ * draw slots as tickets (WORK_QUEUE) or where the CTAs of a row-wise operator beside a tensor-core one take runs of
+ * consecutive blocks: shape[4] / shape[5] = virtual blocks a launched CTA of kernel 1 / 2 takes (1: none, a CTA a slot); shape[1] = CTAs of the kernel resident at once according to cudaOccupancyMaxActiveClusters,
  * which counts one CTA per SM for kernels that allocate tensor memory (0: not asked).
  * shape[2] / shape[3] = 1 when kernel 1 / 2 runs in this fusion with ONE k-slice although it was
  * registered with several: BFUSE_PATTERN_THREAD_SPLIT and BFUSE_PATTERN_WORK_QUEUE cannot host
@@ -146,8 +148,10 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
  * kernel launched through its own handle).
  * out->KernelName points into the context and stays valid until bfuse_destroy. */
 int bfuse_fusion_info(bfuse_context *ctx, int fusion, bfuse_kernel_desc *out);
-/* Which operator and virtual block CTA (or queue ticket) b runs: the if / else-if chain the
+/* Which operator and virtual block dispatch slot b runs: the if / else-if chain the
  * reference prints at the top of a fused kernel (e.g. tests/benchmark/cuda/dense1_0_dense2_6_bfuse.cu:15-63).
+ * A slot is a CTA, or a ticket of the WORK_QUEUE; where CTAs take runs of blocks (bfuse_fusion_info, shape[4..5]) the pattern
+ * deals out runs, and slots are numbered in the order of the launched CTAs, as many to a CTA as its run has blocks.
  * Returns BFUSE_ERR_INVALID for an unmapped b. */
 int bfuse_fusion_map_block(const bfuse_context *ctx, int fusion, int b, int *kernel, int *vblock);
 /* Thread-split fusions: does fused thread t of CTA b run `kernel`?  Fills its virtual ids. */
@@ -187,9 +191,10 @@ int bfuse_launch_list(bfuse_context *ctx, const int *fusions, int n, int mode, v
 int bfuse_graph_create(bfuse_context *ctx, const int *fusions, int n, int mode, int *graph);
 int bfuse_graph_launch(bfuse_context *ctx, int graph, void *stream);
 int bfuse_graph_destroy(bfuse_context *ctx, int graph);
-/* Run the fused grid with a recording body: per CTA the operator, virtual block and SM id it saw
- * (the %smid printf of legacy/tests/thread_pooling_test/temp2.cu:7-9, as data).  Arrays hold
- * fused-grid entries; for WORK_QUEUE they are indexed by ticket.  Synchronises. */
+/* Run the grid of bfuse_launch_fused with a recording body: per dispatch slot the operator, virtual block and SM id its
+ * CTA saw (the %smid printf of legacy/tests/thread_pooling_test/temp2.cu:7-9, as data).  Arrays hold
+ * fused-grid entries indexed by slot as in bfuse_fusion_map_block (by ticket for WORK_QUEUE); -1 where a slot is unused.
+ * Synchronises. */
 int bfuse_trace_fused(bfuse_context *ctx, int fusion, int *kernel_of, int *vblock_of, int *sm_of, int n);
 /* Diagnostic, no reference counterpart: run a registered tcgen05 GEMM kernel once (unfused) with its
  * first CTA recording global-timer marks in nanoseconds: start, set-up done, first / last TMA load
@@ -197,8 +202,8 @@ int bfuse_trace_fused(bfuse_context *ctx, int fusion, int *kernel_of, int *vbloc
  * barrier 1, reduction done, cluster barrier 2, end (12 values; unused marks stay 0). Synchronises. */
 int bfuse_debug_gemm_timeline(bfuse_context *ctx, int kernel, long long *marks, int n);
 /* Diagnostic, no reference counterpart: launch the n block-level fusions back to back on the
- * context's stream (fused mode), every dispatch slot (CTA, or ticket for WORK_QUEUE) of launch i
- * recording three global-timer marks in nanoseconds: kernel entry, body start (the body sets itself
+ * context's stream (fused mode), every dispatch slot (as in bfuse_fusion_map_block; the blocks of a run share their
+ * CTA's marks) of launch i recording three global-timer marks in nanoseconds: kernel entry, body start (the body sets itself
  * up and then waits for the previous launch, so this may precede that launch's end), thread 0 of
  * the body done.  times holds 3 * sum(slots) values,
  * launch i's slots[i] >= its fused grid entries first to last; unused entries stay 0.  Synchronises. */

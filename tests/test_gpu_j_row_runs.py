@@ -34,7 +34,7 @@ def test_runs_equal_one_block_per_cta(rt, row, pattern):
         f = pair.fusion(*pattern)
         info = rt.fusion_info(f)
         assert info["launched_ctas"] < info["GridDim"][0]
-        assert [rt.map_block(f, i)[0] for i in (0, info["GridDim"][0] - 1)] and len(rt.trace_fused(f)[0]) == info["GridDim"][0]
+        assert len(rt.trace_fused(f)[0]) == info["GridDim"][0]
 
 
 def test_runs_of_clusters(rt):
@@ -44,3 +44,36 @@ def test_runs_of_clusters(rt):
     pair = run_and_check(rt, wl.PairSpec("runs", wl.softmax("sm", rng, 7001, 512, 0.125), g, "tf32", "hbm"), [(bf.ZIGZAG, 1, 1), (bf.RANGE_SPLIT, 0, 0)])
     info = rt.fusion_info(pair.fusion(bf.ZIGZAG, 1, 1))
     assert info["launched_ctas"] < info["GridDim"][0]
+
+
+@pytest.mark.parametrize("split", [1, 4])
+@pytest.mark.parametrize("pattern", [(bf.ZIGZAG, 1, 1), (bf.ZIGZAG, 3, 2), (bf.PROPORTIONAL, 3, 0), (bf.SM_STRIPED, 0, 0), (bf.SM_STRIPED, 37, 0),
+                                     (bf.RANGE_SPLIT, 0, 0)])
+def test_slots_describe_the_launch(rt, pattern, split):
+    """Block map, trace and timeline of a launch whose CTAs take runs: every block of both operators in exactly one slot,
+    a run in consecutive slots on one SM with its CTA's time marks, as many CTAs as the fusion says it launches."""
+    rng = np.random.default_rng(13)
+    g = wl.gemm("g", rng, bf.OP_GEMM_TF32, 1, 256, 256, 1024, w_std=0.05, bn=128, split=split)
+    rows = wl.layernorm("ln", rng, 5003, 768, 1e-5)
+    for order in ((rows, g), (g, rows)):
+        pair = run_and_check(rt, wl.PairSpec("runs", *order, "tf32", "hbm"), [pattern])
+        f = pair.fusion(*pattern)
+        info = rt.fusion_info(f)
+        row = order.index(rows)
+        per = info["blocks_per_cta"][row]
+        blocks = [k.launch[0][0] * k.launch[0][1] * k.launch[0][2] for k in order]
+        assert per > 1 and info["blocks_per_cta"][1 - row] == 1 and info["launched_ctas"] < info["GridDim"][0]
+        kern, vb, sm = rt.trace_fused(f)
+        used = sum(blocks)
+        assert (kern[used:] == -1).all() and used <= len(kern) < used + 2 * split
+        for k in range(2):
+            assert sorted(vb[kern == k].tolist()) == list(range(blocks[k]))
+        for i in range(len(kern)):
+            assert rt.map_block(f, i) == (None if i >= used else (int(kern[i]), int(vb[i])))
+        marks = rt.fused_timeline([f])[0]
+        assert (marks[:used] > 0).all() and (marks[:, 0] <= marks[:, 1]).all() and (marks[:, 1] <= marks[:, 2]).all()
+        where = np.nonzero(kern == row)[0]
+        for lo in range(0, blocks[row], per):
+            slots = where[lo:lo + per]      # an operator's blocks are handed out in ascending order
+            assert (np.diff(slots) == 1).all() and (vb[slots] == np.arange(lo, lo + len(slots))).all()
+            assert len(set(sm[slots].tolist())) == 1 and (marks[slots] == marks[slots[0]]).all()

@@ -176,6 +176,39 @@ bool plane_split_ok(int split, int ci) {
 // four; 256 -> 256 on 14 x 14, 32 images, 98 tiles: 38 us with one, 40 with four).
 int plane_split(int tiles, int ci, int share, int sm) { return (long long)tiles * 4 * share <= 2 * sm && plane_split_ok(4, ci) ? 4 : 1; }
 
+// A gathered conv's pixels per tile: the widest of 128 / 64 / 32 that still gives the operator about half the SMs (its
+// pair partner takes the other half); a single small image gets 32-pixel tiles
+int conv_tile_px(const int *s, int ohw, int share, int sm) {
+  for (int cand = kConvBN; cand > 32; cand /= 2)
+    if ((long long)s[0] * ceil_div(ohw, cand) * ceil_div(s[4], kUmmaBM) >= sm / share) return cand;
+  return 32;
+}
+// and its k-slices per tile (a cluster): a deep layer on a small image has few tiles and a long K.  The runtime's own
+// choice is 1 or 4 -- never another width, so that any two operators it tiled can share a launch (a fused launch has one
+// cluster width): 4 when the k-slices still fit three quarters of the SMs and keep at least 4 K blocks each (8-wide
+// clusters measured slower in pairs)
+int conv_k_slices(long long tiles, int num_kb, int share, int sm) { return tiles * 4 * share <= 3 * sm / 2 && num_kb >= 16 ? 4 : 1; }
+
+// Whole planes instead of the gathered form?  Both times are a constant and a time per K block of a k-slice (32 values of
+// k), fitted to 1771 layers of 5 x 5 to 15 x 15 pixels, 32 to 512 channels, stride 1 and 2, batches 1 to 64, alone and two
+// in a launch.  Gathered, microseconds: 5.2 (7.6 in four slices, 0.7 more in a shared launch) + 0.43 a K block with one CTA
+// an SM; with p CTAs an SM 0.44 p, 0.57 p, 0.82 p for 32, 64 and 128 pixels a tile.  Planes: 5.2 + 0.45 (stride 2: 0.52)
+// with one CTA an SM, 1.42 times that for every two; four slices 8.4, or 12.6 with more than one CTA an SM.  The form chosen is the
+// faster of the two within 0.3 % over those layers, never more than 8 % from it: it takes four slices gathered over one of
+// planes (192 -> 128 on 14 x 14, 6 images, alone 15.7 / 28.8 us; 96 -> 64 on 13 x 13, 8 images 12.1 / 17.5), and
+// planes once the gathered tiles crowd the SMs (512 -> 512 on 7 x 7, 8 images 63 / 25; 256 -> 256 on 14 x 14, 32 images 65 / 38).
+bool planes_pay(const int *s, int ohw, int tiles, int split, int share, int sm) {
+  const int bn = conv_tile_px(s, ohw, share, sm), num_kb = ceil_div(s[1] * s[5] * s[6], ConvUmmaTf32::kBK);
+  const long long g_tiles = (long long)s[0] * ceil_div(ohw, bn) * ceil_div(s[4], kUmmaBM);
+  const int g_split = conv_k_slices(g_tiles, num_kb, share, sm);
+  const double g_per = (double)((g_tiles * g_split * share + sm - 1) / sm), g_kb = g_per > 1 ? g_per * (bn == 32 ? 0.44 : bn == 64 ? 0.57 : 0.82) : 0.43;
+  const double gathered = (g_split > 1 ? 7.6 : 5.2) + (share > 1 ? 0.7 : 0.0) + ceil_div(num_kb, g_split) * g_kb;
+  const long long per = ((long long)tiles * split * share + sm - 1) / sm;
+  const double p_kb = (s[7] > 1 ? 0.52 : 0.45) * (per > 1 ? 1.42 * (double)((per + 1) / 2) : 1.0);
+  const double planes = (split == 1 ? 5.2 : per > 1 ? 12.6 : 8.4) + ceil_div(s[1] / 32, split) * 9 * p_kb;
+  return planes < gathered;
+}
+
 int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *err) {
   const int *s = d->shape;
   auto set = [&](int gx, int gy, int gz, int bx, int by, size_t smem, int nargs) {
@@ -231,20 +264,16 @@ int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *
       if (oh <= 0 || ow <= 0) { *err = "conv2d: empty output"; return BFUSE_ERR_SHAPE; }
       const int num_kb = ceil_div(s[1] * s[5] * s[6], ConvUmmaTf32::kBK);
       // Whole planes, shape[11] = 3: 3 x 3 windows on images whose rows the TMA cannot describe, once the batch holds
-      // a whole 128-pixel tile and the gathered form's 32-pixel tiles, split four ways, no longer find an SM each.
-      // Alone, gathered against planes: 512 -> 512 on 7 x 7, 4 images (128 such CTAs) 23.7 / 25.1 us, 8 images
-      // 63 / 25 us, 32 images 123 / 33 us; 256 -> 256 on 14 x 14, 3 images (168 CTAs) 18.5 / 16.9, 32 images 65 / 38 us;
-      // 256 -> 512 with stride 2, 4 images 16.0 / 18.0, 32 images 45 / 24 us.
+      // a whole 128-pixel tile and where planes_pay.
       ConvStaging rows, planes;
-      const long long gathered_ctas = 4LL * s[0] * ceil_div(oh * ow, 32) * ceil_div(s[4], kUmmaBM);
-      if (s[11] == 3 || (s[11] == 0 && s[9] <= 0 && s[10] <= 0 && (long long)s[0] * oh * ow >= kConvBN && gathered_ctas * share > sm &&
+      if (s[11] == 3 || (s[11] == 0 && s[9] <= 0 && s[10] <= 0 && (long long)s[0] * oh * ow >= kConvBN &&
                          !conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, kConvBN, &rows))) {
         const int imgs = conv_plane_staging(s[0], s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, &planes);
         if (!imgs && s[11] == 3) { *err = "conv2d: shape[11] = 3 (whole planes) needs a 3 x 3 window, ci a multiple of 32 and four planes of a tile's images in 16 KB"; return BFUSE_ERR_SHAPE; }
-        if (imgs) {
-          const int px_tiles = ceil_div(s[0] * oh * ow, planes.tile_px), co_tiles = ceil_div(s[4], kUmmaBM), tiles = px_tiles * co_tiles;
-          int split = s[10];
-          if (split <= 0) split = plane_split(tiles, s[1], share, sm);
+        const int px_tiles = imgs ? ceil_div(s[0] * oh * ow, planes.tile_px) : 0, co_tiles = ceil_div(s[4], kUmmaBM), tiles = px_tiles * co_tiles;
+        int split = s[10];
+        if (split <= 0) split = plane_split(tiles, s[1], share, sm);
+        if (imgs && (s[11] == 3 || planes_pay(s, oh * ow, tiles, split, share, sm))) {
           if (!plane_split_ok(split, s[1]) || (s[9] > 0 && s[9] != kConvBN)) { *err = "conv2d: shape[11] = 3 (whole planes) takes 128-pixel tiles and 1, 2, 4 or 8 k-slices of whole groups of 32 channels"; return BFUSE_ERR_SHAPE; }
           const int Kslice = ceil_div(s[1] / 32, split) * 288;
           // two CTAs per SM, whatever the grid
@@ -257,25 +286,15 @@ int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *
           return BFUSE_OK;
         }
       }
-      // pixels per tile: the widest of 128 / 64 / 32 that still gives the operator about half the
-      // SMs (its pair partner takes the other half); a single small image gets 32-pixel tiles
       int bn = s[9];
       if (bn <= 0 && s[11] == 1) bn = kConvBN;   // the staged form has one tile: the 128 lanes of tensor memory
-      if (bn <= 0) {
-        bn = 32;
-        for (int cand = kConvBN; cand > 32; cand /= 2)
-          if ((long long)s[0] * ceil_div(oh * ow, cand) * ceil_div(s[4], kUmmaBM) >= sm / share) { bn = cand; break; }
-      }
+      if (bn <= 0) bn = conv_tile_px(s, oh * ow, share, sm);
       if (bn != 32 && bn != 64 && bn != 128) { *err = "conv2d: pixels per tile must be 32, 64 or 128"; return BFUSE_ERR_SHAPE; }
       d->shape[9] = bn;
       const int K = s[1] * s[5] * s[6];
       const long long tiles = (long long)s[0] * ceil_div(oh * ow, bn) * ceil_div(s[4], kUmmaBM);
-      // k-slices per tile (a cluster): a deep layer on a small image has few tiles and a long K.  The
-      // runtime's own choice is 1 or 4 -- never another width, so that any two operators it tiled can
-      // share a launch (a fused launch has one cluster width): 4 when the k-slices still fit three
-      // quarters of the SMs and keep at least 4 K blocks each (8-wide clusters measured slower in pairs)
       int split = s[10];
-      if (split <= 0) split = (s[11] != 1 && tiles * 4 * share <= 3 * sm / 2 && num_kb >= 16) ? 4 : 1;   // the staged form does not split K
+      if (split <= 0) split = s[11] != 1 ? conv_k_slices(tiles, num_kb, share, sm) : 1;   // the staged form does not split K
       if (split > 8 || split > num_kb) { *err = "conv2d: k-slices must be 1..8 and at most the number of K blocks"; return BFUSE_ERR_SHAPE; }
       const int q = ceil_div(num_kb, split);
       split = ceil_div(num_kb, q);

@@ -116,3 +116,21 @@ def test_lone_long_k_gemm_may_take_two_k_slices():
     down = (1, 512, 4096, 14336, 0, 0, 0)                       # Llama down projection: 224 K blocks in bf16
     assert split(bf.OP_GEMM_BF16, down, 1) == 2 and split(bf.OP_GEMM_BF16, down, 2) in (1, 4)
     assert split(bf.OP_GEMM_TF32, (1, 512, 4096, 4096, 0, 0, 0), 1) == 1      # 128 K blocks: unsplit is as fast
+
+
+def test_whole_planes_are_taken_where_they_are_the_faster_form():
+    """Operand mode and k-slices of 3 x 3 convs whose rows are no 16-byte multiples, alone and as one of a pair; the
+    sizes are ones at which the other form was measured 1.2 to 2 times slower."""
+    def mode(n, ci, hw, co, stride, share):
+        d = bf.KernelDesc()
+        d.KernelName, d.op, d.flags = b"k", bf.OP_CONV2D_TF32, bf.flag_share(share)
+        for i, v in enumerate((n, ci, hw, hw, co, 3, 3, stride, 1)):
+            d.shape[i] = v
+        assert bf.lib().bfuse_default_launch(None, d) == 0
+        return d.shape[11], d.shape[10]
+    for share, shape, want in (
+            (1, (6, 192, 14, 128, 1), (2, 4)), (1, (8, 96, 13, 64, 1), (2, 4)), (1, (24, 192, 14, 128, 2), (2, 4)),   # planes could not split K
+            (2, (12, 192, 7, 128, 1), (2, 4)), (2, (3, 96, 14, 64, 1), (2, 4)), (1, (64, 96, 15, 64, 2), (2, 1)),
+            (1, (8, 512, 7, 512, 1), (3, 4)), (1, (32, 256, 14, 256, 1), (3, 1)), (1, (32, 256, 14, 512, 2), (3, 4)),
+            (2, (4, 256, 14, 256, 1), (3, 4)), (2, (8, 512, 7, 512, 1), (3, 4)), (2, (32, 96, 13, 64, 1), (3, 1))):
+        assert mode(*shape, share) == want, (share, shape)

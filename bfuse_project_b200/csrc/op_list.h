@@ -25,7 +25,7 @@ template <> struct OpAt<4> { using type = GemmSimtF32; };
 template <> struct OpAt<5> { using type = ConvSimtF32; };
 template <> struct OpAt<6> { using type = GemmUmma<0>; };
 template <> struct OpAt<7> { using type = GemmUmma<1>; };
-template <> struct OpAt<8> { using type = ConvUmmaTf32; };
+template <> struct OpAt<8> { using type = ConvAnyTf32; };
 
 struct PairEntry {
   PairLaunchFn block, thread, queue;
@@ -40,7 +40,7 @@ struct PairEntry {
   ClusterCapFn mixed_clusters;
 };
 struct SingleEntry {
-  SingleLaunchFn launch;
+  SingleLaunchFn launch, launch_planes;   // launch_planes: a conv staged as whole planes, else nullptr
   AttrFn attr;
   GroupLaunchFn group;       // up to kGroupMax operators of this body in one launch
   AttrFn group_attr;

@@ -819,9 +819,6 @@ struct ConvUmmaTf32 {
     mark(MARK_END, c.tid == 0);
   }
 
-  // Not inlined: a third form inside run() cost the other two 1 % (batch-256 ResNet branch pair 149.9 -> 151.7 us).
-  __device__ __noinline__ static void run_planes(const Params &p, const TileCtx c) { run_staged<true>(p, c); }
-
   // The sum over the k-slices of a tile whose accumulators hold pixels in their lanes and output channels in
   // their columns; called by every thread of every CTA of the cluster after the MMAs.  The eight 16-channel
   // groups are dealt to the slices round-robin; once the cluster has met (every MMA of the tile is done, so both
@@ -871,8 +868,7 @@ struct ConvUmmaTf32 {
 
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
     if (p.st.slots > 0) {
-      if (p.plane_imgs > 0) run_planes(p, c);
-      else run_staged<false>(p, c);
+      run_staged<false>(p, c);
       return;
     }
     const int warp = c.tid >> 5, lane = c.tid & 31;
@@ -1046,6 +1042,18 @@ struct ConvUmmaTf32 {
       }
     }
     mark(MARK_END, c.tid == 0);
+  }
+};
+
+// All three forms.  A lone gathered or row-staged conv pays for a kernel that holds the call of the third (128 registers
+// instead of 102): 128 -> 128 on 28 x 28, 4 images, 18.7 us without it, 19.8 with; 512 -> 512 on 7 x 7, one image, 21.3 and
+// 22.2.  So lone convs have kernels of both kinds; fused kernels, where the same comparison shows nothing, run this one.
+struct ConvAnyTf32 : ConvUmmaTf32 {
+  // Not inlined: a third form inside run() cost the other two 1 % (batch-256 ResNet branch pair 149.9 -> 151.7 us).
+  __device__ __noinline__ static void run_planes(const Params &p, const TileCtx c) { run_staged<true>(p, c); }
+  __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
+    if (p.plane_imgs > 0) run_planes(p, c);
+    else ConvUmmaTf32::run(p, c);
   }
 };
 

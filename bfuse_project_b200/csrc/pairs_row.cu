@@ -1,6 +1,8 @@
 // One row of the fused-kernel registry: operator BFUSE_ROW fused with every operator.
 #include "op_list.h"
 
+#include <type_traits>
+
 #ifndef BFUSE_ROW
 #error "compile with -DBFUSE_ROW=<operator id>"
 #endif
@@ -67,8 +69,15 @@ template <>
 void fill_pair_row<BFUSE_ROW>(PairEntry *row, SingleEntry *single) {
   using A = typename OpAt<BFUSE_ROW>::type;
   RowFiller<BFUSE_ROW, 0>::fill(row);
-  single->launch = &launch_single<A>;
-  single->attr = &attr_single<A>;
+  if constexpr (std::is_same<A, ConvAnyTf32>::value) {
+    single->launch = &launch_single<ConvUmmaTf32>;
+    single->attr = &attr_single<ConvUmmaTf32>;
+    single->launch_planes = &launch_single<A>;
+  } else {
+    single->launch = &launch_single<A>;
+    single->attr = &attr_single<A>;
+    single->launch_planes = nullptr;
+  }
   single->group = &launch_group<A>;
   single->group_attr = &attr_group<A>;
   single->group_clusters = &clusters_group<A>;

@@ -726,6 +726,9 @@ FusionRec *get_fusion(const bfuse_context *ctx, int h) {
 // Do CTAs of this fusion's launch take runs of virtual blocks (fewer CTAs than dispatch slots)?
 bool takes_runs(const FusionRec &f) { return f.launch.per_cta[0] > 1 || f.launch.per_cta[1] > 1; }
 
+// Is the kernel a conv staged as whole planes?
+bool whole_planes(const KernelRec &k) { return k.desc.op == BFUSE_OP_CONV2D_TF32 && reinterpret_cast<const ConvUmmaParams *>(k.params)->plane_imgs > 0; }
+
 DispatchTable single_table(const bfuse_context *ctx, const KernelRec &k) {
   DispatchTable t;
   std::memset(&t, 0, sizeof(t));
@@ -744,7 +747,8 @@ DispatchTable single_table(const bfuse_context *ctx, const KernelRec &k) {
 int launch_one(bfuse_context *ctx, KernelRec &k, cudaStream_t s) {
   const DispatchTable t = single_table(ctx, k);
   const size_t smem = k.smem + 1024;
-  cudaError_t e = ctx->singles[k.desc.op].launch(t, k.params, (unsigned)k.dims.grid(), (unsigned)k.dims.block(), smem, s);
+  const SingleEntry &se = ctx->singles[k.desc.op];
+  cudaError_t e = (whole_planes(k) ? se.launch_planes : se.launch)(t, k.params, (unsigned)k.dims.grid(), (unsigned)k.dims.block(), smem, s);
   if (e != cudaSuccess) return fail_cuda(ctx, e, ("launch " + k.name).c_str());
   return BFUSE_OK;
 }

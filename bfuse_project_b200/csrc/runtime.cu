@@ -658,6 +658,31 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
   }
 }
 
+// A conv that the runtime staged as whole planes, registered with a launch recorded for its gathered form: that form's
+// GridDim, or a shared-memory window the planes do not fit (they need up to 98 KB, the gathered ring starts at 20 KB).  Such
+// a kernel runs gathered, with what the caller left at the default taken from that form's own launch.
+bool register_gathered(bfuse_context *ctx, KernelRec &k) {
+  bfuse_kernel_desc planes = k.desc, gathered = k.desc;
+  gathered.shape[9] = gathered.shape[10] = 0, gathered.shape[11] = 2;
+  std::string err;
+  if (default_launch(ctx, &planes, &err) || default_launch(ctx, &gathered, &err)) return false;
+  auto same = [](const bfuse_dim3 &a, const bfuse_dim3 &b) { return a.X == b.X && a.Y == b.Y && a.Z == b.Z; };
+  const bool own_window = k.smem == planes.smem_bytes;
+  if (!same(k.desc.GridDim, gathered.GridDim) && (own_window || !same(k.desc.GridDim, planes.GridDim))) return false;
+  std::unique_ptr<KernelRec> alt(new KernelRec(k));
+  std::memcpy(alt->desc.shape, gathered.shape, sizeof(gathered.shape));
+  alt->desc.GridDim = gathered.GridDim;
+  alt->dims.gx = gathered.GridDim.X, alt->dims.gy = gathered.GridDim.Y, alt->dims.gz = gathered.GridDim.Z;
+  alt->smem = alt->desc.smem_bytes = own_window ? gathered.smem_bytes : k.smem;
+  const std::string why = ctx->err;
+  if (build_params(ctx, *alt)) {
+    ctx->err = why;
+    return false;
+  }
+  k = *alt;
+  return true;
+}
+
 __global__ void trace_kernel(const __grid_constant__ DispatchTable t, int *kernel_of, int *vblock_of, int *sm_of) {
   unsigned smid;
   asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
@@ -957,7 +982,7 @@ int bfuse_register_kernel(bfuse_context *ctx, const bfuse_kernel_desc *desc, int
   k->users = 0;
   cudaSetDevice(ctx->device);
   const int rc = build_params(ctx, *k);
-  if (rc) return rc;
+  if (rc && !(rc == BFUSE_ERR_SHAPE && k->desc.op == BFUSE_OP_CONV2D_TF32 && k->desc.shape[11] == 3 && register_gathered(ctx, *k))) return rc;
   *kernel = free_slot(ctx->kernels);
   ctx->kernels[*kernel] = std::move(k);
   return BFUSE_OK;

@@ -56,7 +56,8 @@ enum {
                               /* whole image planes (3 x 3 windows, ci a multiple of 32, tiles of 128 pixels of */
                               /* the whole batch, 1, 2, 4 or 8 k-slices); 0: chosen by bfuse_default_launch  */
                               /* (staged wherever it can be), which writes 1, 2 or 3 back; a kernel          */
-                              /* registered with 0 is gathered                                               */
+                              /* registered with 0 is gathered, and so is one whose 3 was written back and   */
+                              /* that comes with the gathered form's GridDim or a window only that form fits */
   BFUSE_OP_COUNT = 9
 };
 

@@ -79,3 +79,36 @@ def test_ctas_that_walk_several_tiles_and_values_outside_a_window(rt):
     touched[1, 0, :2, :2] = True
     assert torch.equal(outs[2][~touched.expand_as(outs[2])], outs[0][~touched.expand_as(outs[0])])
     assert not torch.isfinite(outs[2][1, :, :2, :2]).any()
+
+
+@pytest.mark.parametrize("n,ci,hw,co,stride", [(8, 256, 14, 256, 1), (32, 64, 7, 96, 2), (32, 256, 14, 40, 1)])
+def test_a_launch_recorded_for_the_gathered_form_is_still_accepted(rt, n, ci, hw, co, stride):
+    """The runtime's choice is whole planes; a window too small for them, the gathered form's grid, or both register and run gathered."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    x = torch.randn(n, ci, hw, hw, device="cuda", generator=g)
+    w = torch.randn(co, ci, 3, 3, device="cuda", generator=g) * 0.05
+    o = (hw - 1) // stride + 1
+    shape = (n, ci, hw, hw, co, 3, 3, stride, 1)
+    # (registered at once: the planes' own launch and one that fits neither form)
+    planes = rt.describe("c", bf.OP_CONV2D_TF32, shape + (128, 0, 3))
+    gathered = rt.describe("c", bf.OP_CONV2D_TF32, shape + (0, 0, 2))
+
+    def run(**launch):
+        y = torch.zeros(n, co, o, o, device="cuda")
+        sh = (0, 0, 2) if launch.pop("mode", 0) == 2 else (128, planes.shape[10], 3)
+        k = rt.register_kernel(rt.describe("c", bf.OP_CONV2D_TF32, shape + sh, [x.data_ptr(), w.data_ptr(), y.data_ptr()], **launch))
+        rt.launch_kernel(k)
+        assert rt.read_status() == 0
+        return y
+    want = run(mode=2)
+    grid = gathered.GridDim.tuple()
+    for launch in (dict(smem=gathered.smem_bytes), dict(grid=grid), dict(grid=grid, smem=gathered.smem_bytes)):
+        if launch.get("grid") and grid[0] * grid[1] * grid[2] <= planes.GridDim.size():
+            continue   # a grid the planes can walk as it is
+        assert torch.equal(run(**launch), want), launch
+    for launch in (dict(smem=4096), dict(grid=(grid[0] + 1, grid[1], grid[2] + 1))):
+        with pytest.raises(bf.BfuseError) as err:
+            run(**launch)
+        assert err.value.code == 2

@@ -794,7 +794,14 @@ bool ring_info(const KernelRec &k, int *header, int *stage_bytes, int *min_stage
     const int bn = s[9] > 0 ? s[9] : kConvBN;
     const ConvUmmaParams *cp = reinterpret_cast<const ConvUmmaParams *>(k.params);
     const int K = s[1] * s[5] * s[6];
-    if (cp->plane_imgs) return false;   // whole planes: weight and A stages share their barriers, four of each
+    if (cp->plane_imgs) {
+      // whole planes: raw slots can be given up, the four weight stages share their barriers with the A stages (the raw
+      // ring is rounded up to 1 KB; slots are multiples of 128 bytes)
+      *header = kUmmaHeaderBytes + kConvAStages * kUmmaABytes + 1024 - 128, *stage_bytes = cp->st.slot_pitch;
+      *min_stages = std::min(2, cp->kb_per_slice * ConvUmmaTf32::kBK / (9 * cp->st.cc));
+      *stages = cp->st.slots;
+      return true;
+    }
     if (cp->st.slots) {   // staged: the raw ring stays as registered, the 16 KB weight stages are what can be given up
       *header = conv_header_bytes(K) + conv_raw_bytes(cp->st.slots, cp->st.slot_pitch), *stage_bytes = kUmmaABytes;
       *min_stages = std::min(2, K / ConvUmmaTf32::kBK);
@@ -812,9 +819,34 @@ bool ring_info(const KernelRec &k, int *header, int *stage_bytes, int *min_stage
 const void *params_with_stages(const KernelRec &k, int stages, unsigned char *scratch) {
   if (stages <= 0) return k.params;
   std::memcpy(scratch, k.params, kParamsBytes);
-  if (k.desc.op == BFUSE_OP_CONV2D_TF32) reinterpret_cast<ConvUmmaParams *>(scratch)->stages = stages;
+  if (whole_planes(k)) reinterpret_cast<ConvUmmaParams *>(scratch)->st.slots = stages;
+  else if (k.desc.op == BFUSE_OP_CONV2D_TF32) reinterpret_cast<ConvUmmaParams *>(scratch)->stages = stages;
   else reinterpret_cast<GemmUmmaParams *>(scratch)->stages = stages;
   return scratch;
+}
+
+// A hidden record of registered kernel `reg` tiled with one k-slice, the same buffers: `gathered` turns a conv staged as
+// whole planes to the gathered form.
+int add_unsplit(bfuse_context *ctx, int reg, bool gathered, int *slot) {
+  const KernelRec &orig = *ctx->kernels[reg];
+  std::unique_ptr<KernelRec> alt(new KernelRec(orig));
+  const bool conv = orig.desc.op == BFUSE_OP_CONV2D_TF32;
+  alt->desc.shape[conv ? 10 : 5] = 1;
+  if (!conv) alt->desc.shape[6] = 0;   // tile height: the runtime's choice for the unsplit form
+  if (gathered) alt->desc.shape[9] = 0, alt->desc.shape[11] = 2;
+  alt->desc.KernelName = nullptr;
+  std::string err;
+  int rc = default_launch(ctx, &alt->desc, &err);
+  if (rc) return fail(ctx, rc, orig.name + " (re-tiled with one k-slice): " + err);
+  alt->dims = {alt->desc.GridDim.X, alt->desc.GridDim.Y, alt->desc.GridDim.Z, alt->desc.BlockDim.X, alt->desc.BlockDim.Y, alt->desc.BlockDim.Z};
+  alt->smem = alt->desc.smem_bytes;
+  alt->alias_of = reg;
+  alt->users = 0;
+  rc = build_params(ctx, *alt);
+  if (rc) return rc;
+  *slot = free_slot(ctx->kernels);
+  ctx->kernels[*slot] = std::move(alt);
+  return BFUSE_OK;
 }
 
 int launch_fused_rec(bfuse_context *ctx, FusionRec &f, cudaStream_t s, const DispatchTable *table = nullptr) {
@@ -1035,35 +1067,34 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
         if (x >= 0 && !keep) c->kernels[x].reset();
     }
   } undo{ctx};
-  if (pattern == PATTERN_THREAD_SPLIT || pattern == PATTERN_WORK_QUEUE) {
-    KernelRec **side[2] = {&a, &b};
-    int *handle[2] = {&f->k1, &f->k2};
-    for (int i = 0; i < 2; ++i) {
-      KernelRec *orig = *side[i];
-      if (orig->cluster <= 1) continue;
-      std::unique_ptr<KernelRec> alt(new KernelRec(*orig));
-      const bool conv = orig->desc.op == BFUSE_OP_CONV2D_TF32;
-      alt->desc.shape[conv ? 10 : 5] = 1;
-      if (!conv) alt->desc.shape[6] = 0;   // tile height: the runtime's choice for the unsplit form
-      alt->desc.KernelName = nullptr;
-      std::string err;
-      int rc = default_launch(ctx, &alt->desc, &err);
-      if (rc) return fail(ctx, rc, orig->name + " (re-tiled with one k-slice): " + err);
-      alt->dims = {alt->desc.GridDim.X, alt->desc.GridDim.Y, alt->desc.GridDim.Z, alt->desc.BlockDim.X, alt->desc.BlockDim.Y, alt->desc.BlockDim.Z};
-      alt->smem = alt->desc.smem_bytes;
-      alt->alias_of = *handle[i];
-      alt->users = 0;
-      rc = build_params(ctx, *alt);
-      if (rc) return rc;
-      const int slot = free_slot(ctx->kernels);
-      ctx->kernels[slot] = std::move(alt);
-      undo.h[i] = slot;
-      *handle[i] = slot;
-      *side[i] = ctx->kernels[slot].get();
-      f->retiled[i] = true;
-    }
-    // free_slot may have grown the table: the unique_ptrs moved, the records they own did not
-    a = ctx->kernels[f->k1].get(), b = ctx->kernels[f->k2].get();
+  KernelRec **side[2] = {&a, &b};
+  int *handle[2] = {&f->k1, &f->k2};
+  const int reg[2] = {kernel1, kernel2};
+  auto retile = [&](int i, bool gathered) {
+    int slot;
+    const int rc = add_unsplit(ctx, reg[i], gathered, &slot);
+    if (rc) return rc;
+    if (undo.h[i] >= 0) ctx->kernels[undo.h[i]].reset();   // it was re-tiled once already
+    undo.h[i] = *handle[i] = slot;
+    *side[i] = ctx->kernels[slot].get();   // (the table may have grown: the unique_ptrs moved, the records they own did not)
+    f->retiled[i] = true;
+    return (int)BFUSE_OK;
+  };
+  if (pattern == PATTERN_THREAD_SPLIT || pattern == PATTERN_WORK_QUEUE)
+    for (int i = 0; i < 2; ++i)
+      if ((*side[i])->cluster > 1)
+        if (const int rc = retile(i, false)) return rc;
+  // Thread split lays the two windows side by side; whole planes, whose window cannot go below four weight stages and
+  // two raw slots (up to 98 KB), give way to the gathered form where the sum does not fit with the rings at their shallowest.
+  if (pattern == PATTERN_THREAD_SPLIT) {
+    auto least = [](const KernelRec &k) {
+      int hdr, stg, mn, st;
+      const size_t w = ring_info(k, &hdr, &stg, &mn, &st) ? (size_t)hdr + (size_t)std::min(mn, st) * stg : k.smem;
+      return (std::min(w, k.smem) + 1023) / 1024 * 1024;
+    };
+    for (int i = 0; i < 2; ++i)
+      if (whole_planes(**side[i]) && least(*a) + least(*b) + 1024 > kMaxSmemPerCta)
+        if (const int rc = retile(i, true)) return rc;
   }
   const KernelDims kd[2] = {a->dims, b->dims};
   if (pattern == PATTERN_SM_STRIPED && param_m == 0) param_m = ctx->sm_count;

@@ -4,6 +4,7 @@ import pytest
 
 import bfuse_project_b200 as bf
 from bfuse_project_b200 import workloads as wl
+from pair_oracle import check_against_oracle
 from test_gpu_b_pairs import BLOCK_PATTERNS, run_and_check
 
 pytestmark = pytest.mark.gpu
@@ -112,3 +113,28 @@ def test_a_launch_recorded_for_the_gathered_form_is_still_accepted(rt, n, ci, hw
         with pytest.raises(bf.BfuseError) as err:
             run(**launch)
         assert err.value.code == 2
+
+
+def test_thread_split_beside_a_wide_window(rt):
+    """Thread split lays both windows side by side: the planes' raw slots are given up first, and where even two of them do
+    not fit beside the partner the conv runs gathered, as the fusion's own sequential mode does."""
+    rng = np.random.default_rng(21)
+    planes = wl.conv2d("planes", rng, bf.OP_CONV2D_TF32, 5, 128, 14, 14, 64, 3, 1, 1, bn=128, split=1, mode=3)
+    rows = wl.conv2d("rows", rng, bf.OP_CONV2D_TF32, 2, 512, 28, 28, 128, 3, 1, 1, bn=128, split=1, mode=1)
+    for smem, retiled in ((130 * 1024, False), (200 * 1024, True)):
+        rows.smem = smem
+        for order in ((planes, rows), (rows, planes)):
+            pair = wl.DevicePair(rt, wl.PairSpec("wide", *order, "tf32", "hbm"))
+            f = pair.fusion(bf.THREAD_SPLIT, 0, 0)
+            info = rt.fusion_info(f)
+            assert any(info["retiled_unsplit"]) == retiled, (smem, info)
+            pair.clear_outputs()
+            rt.launch_sequential(f)
+            want = pair.read_outputs()
+            pair.clear_outputs()
+            rt.launch_fused(f)
+            got = pair.read_outputs()
+            assert rt.read_status() == 0
+            for k, ks in enumerate(order):
+                assert np.array_equal(want[k][0], got[k][0]), (smem, ks.name)
+                check_against_oracle(ks, got[k], ks.name)

@@ -65,7 +65,7 @@ struct FusionRec {
 
 struct GroupRec {
   int n;
-  int ks[kGroupMax];
+  int ks[kGroupMax], reg[kGroupMax];   // the kernels it launches (hidden unsplit re-tilings where they differ) and was registered with
   GroupPlan plan;
   std::string name;
   size_t smem;
@@ -849,6 +849,16 @@ int add_unsplit(bfuse_context *ctx, int reg, bool gathered, int *slot) {
   return BFUSE_OK;
 }
 
+// One cluster width a launch: may this kernel give up its k-slices beside an operator of another width?  A conv that the
+// runtime would have left unsplit in the gathered form, but splits as whole planes.
+bool slices_optional(const bfuse_context *ctx, const KernelRec &k) {
+  if (!whole_planes(k) || k.cluster <= 1) return false;
+  bfuse_kernel_desc gathered = k.desc;
+  gathered.shape[9] = gathered.shape[10] = 0, gathered.shape[11] = 2;
+  std::string err;
+  return default_launch(ctx, &gathered, &err) == BFUSE_OK && gathered.shape[10] == 1;
+}
+
 int launch_fused_rec(bfuse_context *ctx, FusionRec &f, cudaStream_t s, const DispatchTable *table = nullptr) {
   KernelRec &a = *ctx->kernels[f.k1], &b = *ctx->kernels[f.k2];
   const PairEntry &pe = ctx->pairs[a.desc.op][b.desc.op];
@@ -1096,6 +1106,9 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
       if (whole_planes(**side[i]) && least(*a) + least(*b) + 1024 > kMaxSmemPerCta)
         if (const int rc = retile(i, true)) return rc;
   }
+  for (int i = 0; i < 2; ++i)
+    if (a->cluster != b->cluster && a->cluster > 1 && b->cluster > 1 && slices_optional(ctx, **side[i]))
+      if (const int rc = retile(i, false)) return rc;
   const KernelDims kd[2] = {a->dims, b->dims};
   if (pattern == PATTERN_SM_STRIPED && param_m == 0) param_m = ctx->sm_count;
   if (pattern != PATTERN_SM_STRIPED && pattern != PATTERN_THREAD_SPLIT && pattern != PATTERN_RANGE_SPLIT) {
@@ -1255,10 +1268,29 @@ int bfuse_register_group(bfuse_context *ctx, const int *kernels, int n, int patt
   for (int i = 0; i < n; ++i) {
     ks[i] = get_kernel(ctx, kernels[i]);
     if (!ks[i] || ks[i]->alias_of >= 0) return fail(ctx, BFUSE_ERR_INVALID, "bad kernel handle");
-    g->ks[i] = kernels[i];
+    g->ks[i] = g->reg[i] = kernels[i];
+    g->name += (i ? "_" : "") + ks[i]->name;
+  }
+  struct Undo {   // hidden records are dropped again if the registration fails further down
+    bfuse_context *c;
+    int h[kGroupMax] = {-1, -1, -1, -1};
+    bool keep = false;
+    ~Undo() {
+      for (int x : h)
+        if (x >= 0 && !keep) c->kernels[x].reset();
+    }
+  } undo{ctx};
+  int narrow = 0, wide = 0;   // cluster widths above 1
+  for (int i = 0; i < n; ++i)
+    if (ks[i]->cluster > 1) narrow = narrow ? std::min(narrow, ks[i]->cluster) : ks[i]->cluster, wide = std::max(wide, ks[i]->cluster);
+  for (int i = 0; i < n; ++i) {
+    if (narrow != wide && slices_optional(ctx, *ks[i])) {
+      if (const int rc = add_unsplit(ctx, kernels[i], false, &undo.h[i])) return rc;
+      g->ks[i] = undo.h[i];
+      ks[i] = ctx->kernels[undo.h[i]].get();
+    }
     kd[i] = ks[i]->dims;
     cluster = std::max(cluster, ks[i]->cluster);
-    g->name += (i ? "_" : "") + ks[i]->name;
   }
   g->name += "_fused_bfuse";
   // one body, or two: a kernel exists per body and per unordered pair of bodies
@@ -1321,7 +1353,8 @@ int bfuse_register_group(bfuse_context *ctx, const int *kernels, int n, int patt
   cudaError_t e = mixed ? mixed_entry.mixed_attr(&attr) : ctx->singles[ks[0]->desc.op].group_attr(&attr);
   if (e != cudaSuccess) return fail_cuda(ctx, e, "cudaFuncGetAttributes");
   g->regs = attr.numRegs;
-  for (int i = 0; i < n; ++i) ++ks[i]->users;
+  undo.keep = true;
+  for (int i = 0; i < n; ++i) ++ctx->kernels[g->reg[i]]->users;
   *group = free_slot(ctx->groups);
   ctx->groups[*group] = std::move(g);
   return BFUSE_OK;
@@ -1556,7 +1589,10 @@ int bfuse_unregister_fusion(bfuse_context *ctx, int fusion) {
 int bfuse_unregister_group(bfuse_context *ctx, int group) {
   GroupRec *g = get_group(ctx, group);
   if (!g) return fail(ctx, BFUSE_ERR_INVALID, "bad group handle");
-  for (int i = 0; i < g->n; ++i) --ctx->kernels[g->ks[i]]->users;
+  for (int i = 0; i < g->n; ++i) {
+    --ctx->kernels[g->reg[i]]->users;
+    if (g->ks[i] != g->reg[i]) ctx->kernels[g->ks[i]].reset();
+  }
   ctx->groups[group].reset();
   return BFUSE_OK;
 }

@@ -144,7 +144,8 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
  * which counts one CTA per SM for kernels that allocate tensor memory (0: not asked).
  * shape[2] / shape[3] = 1 when kernel 1 / 2 runs in this fusion with ONE k-slice although it was
  * registered with several, or gathered although it was staged as whole planes (a thread split whose
- * windows do not fit side by side otherwise): BFUSE_PATTERN_THREAD_SPLIT and BFUSE_PATTERN_WORK_QUEUE cannot host
+ * windows do not fit side by side otherwise); a conv whose k-slices only the whole-plane form brought gives them up
+ * beside an operator of another cluster width, in groups too: BFUSE_PATTERN_THREAD_SPLIT and BFUSE_PATTERN_WORK_QUEUE cannot host
  * operators launched as thread-block clusters, so such an operator is re-tiled unsplit for the fusion
  * (all launch modes of the fusion use that tiling; its sums differ in the last bits from the k-split
  * kernel launched through its own handle).

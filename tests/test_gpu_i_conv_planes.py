@@ -138,3 +138,38 @@ def test_thread_split_beside_a_wide_window(rt):
             for k, ks in enumerate(order):
                 assert np.array_equal(want[k][0], got[k][0]), (smem, ks.name)
                 check_against_oracle(ks, got[k], ks.name)
+
+
+def test_planes_beside_an_operator_of_another_cluster_width(rt):
+    """The runtime splits this conv in four slices as whole planes and would leave it unsplit gathered: beside a GEMM of two
+    k-slices it runs in one, as a pair and in a group, and the records it needs for that are released with them."""
+    rng = np.random.default_rng(22)
+    conv = wl.conv2d("planes", rng, bf.OP_CONV2D_TF32, 8, 256, 14, 14, 256, 3, 1, 1)
+    gemm = wl.gemm("g", rng, bf.OP_GEMM_TF32, 1, 100, 64, 1024, w_std=0.05, bn=64, split=2)
+    pair = wl.DevicePair(rt, wl.PairSpec("widths", conv, gemm, "tf32", "hbm"))
+    f = pair.fusion(bf.ZIGZAG, 1, 1)
+    assert rt.fusion_info(f)["retiled_unsplit"] == (True, False)
+    pair.clear_outputs()
+    rt.launch_sequential(f)
+    want = pair.read_outputs()
+    check_against_oracle(conv, want[0], "planes")
+    check_against_oracle(gemm, want[1], "gemm")
+    g = rt.register_group([pair.kernels[1], pair.kernels[0]], bf.ZIGZAG, 1, 1)
+    for launch in (lambda: rt.launch_fused(f), lambda: rt.launch_group(g)):
+        pair.clear_outputs()
+        launch()
+        got = pair.read_outputs()
+        assert rt.read_status() == 0
+        assert np.array_equal(got[0][0], want[0][0]) and np.array_equal(got[1][0], want[1][0])
+    with pytest.raises(bf.BfuseError):
+        rt.unregister_kernel(pair.kernels[0])
+    rt.unregister_group(g)
+    rt.unregister_fusion(pair.fusions.pop((bf.ZIGZAG, 1, 1)))
+    for k in pair.kernels:
+        rt.unregister_kernel(k)
+    # an explicit width that the gathered form would not have come without stays refused
+    four = wl.conv2d("four", rng, bf.OP_CONV2D_TF32, 1, 512, 7, 7, 64, 3, 1, 1)
+    pair = wl.DevicePair(rt, wl.PairSpec("widths", four, gemm, "tf32", "hbm"))
+    with pytest.raises(bf.BfuseError) as err:
+        pair.fusion(bf.ZIGZAG, 1, 1)
+    assert err.value.code == 7

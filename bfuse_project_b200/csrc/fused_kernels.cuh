@@ -405,6 +405,10 @@ template <class A, class B>
 int clusters_block_pair_wide(unsigned block, size_t smem, int cluster) {
   return max_resident_clusters(fused_block_kernel<A, B, pair_wide_blocks<A, B>()>, block, smem, cluster);
 }
+template <class A, class B>
+int clusters_queue_pair(unsigned block, size_t smem, int cluster) {
+  return max_resident_clusters(fused_queue_kernel<A, B>, block, smem, cluster);
+}
 template <class A>
 int clusters_group(unsigned block, size_t smem, int cluster) {
   return max_resident_clusters(fused_group_kernel<A>, block, smem, cluster);

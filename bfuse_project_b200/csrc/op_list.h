@@ -33,7 +33,7 @@ struct PairEntry {
   PairLaunchFn block_wide;   // the register-richer build of the pair (see pair_wide_blocks), else nullptr
   AttrFn block_wide_attr;
   int wide_min_blocks;       // CTAs per SM the wide build is compiled for
-  ClusterCapFn block_clusters;  // clusters of the block-level kernel that can be resident at once
+  ClusterCapFn block_clusters, block_wide_clusters, queue_clusters;  // clusters of the kernel that can be resident at once
   // groups of these two bodies (built once per unordered pair: for row < column only, else nullptr)
   MixedGroupLaunchFn mixed;
   AttrFn mixed_attr;

@@ -14,6 +14,7 @@ struct WideFiller {
   static void fill(PairEntry &e) {
     e.block_wide = nullptr;
     e.block_wide_attr = nullptr;
+    e.block_wide_clusters = nullptr;
     e.wide_min_blocks = 0;
   }
 };
@@ -22,6 +23,7 @@ struct WideFiller<A, B, true> {
   static void fill(PairEntry &e) {
     e.block_wide = &launch_block_pair_wide<A, B>;
     e.block_wide_attr = &attr_block_pair_wide<A, B>;
+    e.block_wide_clusters = &clusters_block_pair_wide<A, B>;
     e.wide_min_blocks = pair_wide_blocks<A, B>();
   }
 };
@@ -55,6 +57,7 @@ struct RowFiller {
     row[J].thread_attr = &attr_thread_pair<A, B>;
     row[J].queue_attr = &attr_queue_pair<A, B>;
     row[J].block_clusters = &clusters_block_pair<A, B>;
+    row[J].queue_clusters = &clusters_queue_pair<A, B>;
     WideFiller<A, B, (pair_wide_blocks<A, B>() > 0)>::fill(row[J]);
     MixedFiller<A, B, (I < J)>::fill(row[J]);
     RowFiller<I, J + 1>::fill(row);

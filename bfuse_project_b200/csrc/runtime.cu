@@ -1438,17 +1438,18 @@ int bfuse_fusion_info(bfuse_context *ctx, int fusion, bfuse_kernel_desc *out) {
   out->op = -1;
   out->smem_bytes = f->smem;
   out->shape[0] = (int)f->launch_grid;  // CTAs actually launched (fewer than GridDim for the work queue and for runs of blocks)
-  // CTAs of this kernel resident at once according to the occupancy calculator (whole clusters; one CTA per SM
-  // for kernels that allocate tensor memory), 0 when not asked
+  // CTAs of this kernel -- the build that is launched -- resident at once according to the occupancy calculator (whole
+  // clusters; one CTA per SM for kernels that allocate tensor memory), 0 for thread split, where it is not asked
   out->shape[1] = 0;
   // operator 1 / 2 runs here in a one-k-slice re-tiling of the registered kernel (thread split, work queue)
   out->shape[2] = f->retiled[0] ? 1 : 0;
   out->shape[3] = f->retiled[1] ? 1 : 0;
   for (int i = 0; i < 2; ++i) out->shape[4 + i] = std::max(1, f->launch.per_cta[i]);   // virtual blocks a launched CTA takes
-  if (f->plan.table.kind != DISPATCH_THREADS && !f->wide) {
+  if (f->plan.table.kind != DISPATCH_THREADS) {
     const int cl = std::max(1, f->plan.table.cluster);
     cudaSetDevice(ctx->device);
-    const int cap = ctx->pairs[ctx->kernels[f->k1]->desc.op][ctx->kernels[f->k2]->desc.op].block_clusters((unsigned)f->plan.fused_block, f->smem, cl);
+    const PairEntry &pe = ctx->pairs[ctx->kernels[f->k1]->desc.op][ctx->kernels[f->k2]->desc.op];
+    const int cap = (f->plan.table.queue ? pe.queue_clusters : f->wide ? pe.block_wide_clusters : pe.block_clusters)((unsigned)f->plan.fused_block, f->smem, cl);
     if (cap > 0) out->shape[1] = cap * cl;
   }
   return BFUSE_OK;

@@ -140,8 +140,8 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
  * name "<k1>_<k2>_fused_{bfuse,hfuse}", fused GridDim / BlockDim, plus smem and registers;
  * GridDim counts the pattern's dispatch slots, one virtual block each; shape[0] = CTAs launched, fewer where persistent CTAs
  * draw slots as tickets (WORK_QUEUE) or where the CTAs of a row-wise operator beside a tensor-core one take runs of
- * consecutive blocks: shape[4] / shape[5] = virtual blocks a launched CTA of kernel 1 / 2 takes (1: none, a CTA a slot); shape[1] = CTAs of the kernel resident at once according to cudaOccupancyMaxActiveClusters,
- * which counts one CTA per SM for kernels that allocate tensor memory (0: not asked).
+ * consecutive blocks: shape[4] / shape[5] = virtual blocks a launched CTA of kernel 1 / 2 takes (1: none, a CTA a slot); shape[1] = CTAs of the launched kernel resident at once according to cudaOccupancyMaxActiveClusters,
+ * which counts one CTA per SM for kernels that allocate tensor memory (0: not asked, thread split).
  * shape[2] / shape[3] = 1 when kernel 1 / 2 runs in this fusion with ONE k-slice although it was
  * registered with several, or gathered although it was staged as whole planes (a thread split whose
  * windows do not fit side by side otherwise); a conv whose k-slices only the whole-plane form brought gives them up

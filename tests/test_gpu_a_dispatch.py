@@ -122,3 +122,18 @@ def test_which_operators_share_an_sm(rt):
     assert all(len(set((np.nonzero(sm == s)[0] % 2).tolist())) <= 1 for s in range(rt.sm_count))   # an SM sees CTAs of one parity
     _, kern, sm = sms_with_both(bf.RANGE_SPLIT, 0, 0)
     assert set(kern[:rt.sm_count].tolist()) == {0}
+
+
+def test_residency_is_that_of_the_launched_build(rt, pair):
+    """Two row-wise operators have three block-level builds of different register counts; the residency a fusion reports is the one its
+    registers allow the build it launches (65 536 an SM, eight to a thread at a time, a warp's in units of 256)."""
+    def by_regs(info):
+        per_warp = -(-info["Reg"] // 8) * 8 * 32
+        return rt.sm_count * min(2048 // info["BlockDim"][0], 65536 // (per_warp * (info["BlockDim"][0] // 32)))
+    small = wl.DevicePair(rt, wl.make_pair("cfg1_softmax_layernorm", seed=2, scale=0.25))
+    seen = set()
+    for p, pattern in ((pair, bf.ZIGZAG), (small, bf.ZIGZAG), (pair, bf.WORK_QUEUE)):
+        info = rt.fusion_info(p.fusion(pattern, 1, 1))
+        assert info["resident_ctas"] == by_regs(info), info
+        seen.add((info["Reg"], info["resident_ctas"]))
+    assert len(seen) > 1

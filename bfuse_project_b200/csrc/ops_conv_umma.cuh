@@ -117,6 +117,7 @@ __host__ __device__ inline int conv_plane_staging(int n, int ci, int h, int wd, 
   // (slots start 2 KB into the window and 16 KB of weights follow the last one: a tap up to two rows outside
   // its plane stays inside the window)
   if (kh != 3 || kw != 3 || ci % 32 || pad > 2 || wd > 64) return 0;
+  if ((long long)n * oh * ow > 0x7fffffff - kConvBN) return 0;   // pixels are counted over the batch, in 32 bits
   const int ohw = oh * ow;
   // 128 consecutive pixels of the batch touch up to `span` images; where their planes would leave the raw ring
   // fewer than six slots, tiles of whole images (49-pixel outputs of a 14 x 14 input: two instead of four)

@@ -134,3 +134,11 @@ def test_whole_planes_are_taken_where_they_are_the_faster_form():
             (1, (8, 512, 7, 512, 1), (3, 4)), (1, (32, 256, 14, 256, 1), (3, 1)), (1, (32, 256, 14, 512, 2), (3, 4)),
             (2, (4, 256, 14, 256, 1), (3, 4)), (2, (8, 512, 7, 512, 1), (3, 4)), (2, (32, 96, 13, 64, 1), (3, 1))):
         assert mode(*shape, share) == want, (share, shape)
+
+
+def test_batches_whose_pixels_do_not_fit_32_bits_are_gathered():
+    """Whole planes count output pixels over the batch; the gathered form counts them by image and takes any batch."""
+    few = default(bf.OP_CONV2D_TF32, (200_000_000, 32, 1, 1, 8, 3, 3, 1, 2))     # 9 pixels an image
+    many = default(bf.OP_CONV2D_TF32, (240_000_000, 32, 1, 1, 8, 3, 3, 1, 2))
+    assert few.shape[11] == 3 and few.GridDim.tuple() == (296, 1, 1)
+    assert many.shape[11] == 2 and many.GridDim.tuple() == (1, 1, 240_000_000)

@@ -1722,6 +1722,12 @@ int bfuse_debug_conv_staging(const int *shape, int bn, int *out, int n) {
   const int oh = conv_out(s[2], s[5], s[7], s[8]), ow = conv_out(s[3], s[6], s[7], s[8]);
   ConvStaging st;
   std::memset(&st, 0, sizeof(st));
+  if (bn == 0) {
+    const int imgs = oh > 0 && ow > 0 ? conv_plane_staging(s[0], s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, &st) : 0;
+    const int v[13] = {imgs, st.cc, st.rows, st.pitch, st.ex, st.ey, st.step_x, st.step_y, st.x_start, st.x_off, st.slot_bytes, st.slot_pitch, st.tile_px};
+    std::memcpy(out, v, sizeof(int) * (n >= 13 ? 13 : 12));
+    return BFUSE_OK;
+  }
   const bool ok = oh > 0 && ow > 0 && conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, bn, &st);
   const int v[13] = {ok ? st.slots : 0, st.cc, st.rows, st.pitch, st.ex, st.ey, st.step_x, st.step_y, st.x_start, st.x_off, st.slot_bytes, st.slot_pitch,
                      st.tile_px};

@@ -98,3 +98,49 @@ def test_what_cannot_be_staged():
     assert staging((1, 64, 56, 56, 128, 3, 3, 2, 1), 64)["slots"] == 0       # the tile is the 128 lanes of tensor memory
     assert staging((1, 12, 20, 20, 200, 3, 3, 1, 1), 128)["slots"] == 0      # K = 108: no whole number of K blocks
     assert staging((1, 64, 56, 56, 128, 3, 3, 2, 1), 128)["slots"] == 3
+
+
+PLANES = [(3, 64, 7, 7, 3, 3, 1, 1), (32, 64, 7, 7, 3, 3, 1, 1), (5, 32, 14, 14, 3, 3, 2, 1), (9, 32, 14, 14, 3, 3, 1, 1), (11, 64, 5, 5, 3, 3, 1, 0),
+          (9, 96, 10, 10, 3, 3, 2, 2), (9, 96, 13, 13, 3, 3, 1, 2), (4, 32, 15, 9, 3, 3, 1, 1), (2, 32, 3, 50, 3, 3, 1, 1), (40, 64, 15, 15, 3, 3, 2, 1)]
+
+
+@pytest.mark.parametrize("shape", PLANES)
+def test_whole_planes_equal_im2col(shape):
+    """Whole planes replayed: every tile's raw slots hold the images the tile's pixels touch, copied contiguously from 16-byte
+    boundaries; the window origin of a pixel plus a tap's offset is the im2col element where the tap lies inside the
+    image, and where it does not the body masks it and the address stays within two rows of the slot."""
+    n, ci, h, w, kh, kw, stride, pad = shape
+    st = staging((n, ci, h, w, 128, kh, kw, stride, pad), 0)
+    imgs, cc, tile = st["slots"], st["cc"], st["tile_px"]
+    assert imgs > 0 and cc % 4 == 0 and 32 % cc == 0 and 0 < tile <= 128 and (st["rows"], st["pitch"]) == (h, w)
+    assert st["slot_bytes"] == cc * h * w * 4 and st["slot_bytes"] % 16 == 0 and st["slot_pitch"] >= imgs * st["slot_bytes"] and st["slot_pitch"] <= 16 * 1024 + 127
+    oh, ow = (h + 2 * pad - kh) // stride + 1, (w + 2 * pad - kw) // stride + 1
+    ohw, total = oh * ow, n * oh * ow
+    x = np.random.default_rng(3).standard_normal((n, ci, h, w)).astype(np.float32)
+    padded = np.zeros((n, cc, h + 2 * pad, w + 2 * pad), np.float32)
+    for c0 in (0, ci - cc):
+        assert c0 * h * w * 4 % 16 == 0 and ci * h * w * 4 % 16 == 0     # where a slot's copies start
+        padded[:, :, pad:pad + h, pad:pad + w] = x[:, c0:c0 + cc]
+        for px0 in range(0, total, tile):
+            px = np.arange(px0, min(px0 + tile, total))
+            img0 = px0 // ohw
+            assert px[-1] // ohw - img0 + 1 <= imgs
+            slot = np.concatenate([x[i, c0:c0 + cc].reshape(-1) for i in range(img0, px[-1] // ohw + 1)])
+            img, oy, ox = px // ohw, px % ohw // ow, px % ohw % ow
+            iy, ix = oy * st["step_y"] + st["x_off"], ox * st["step_x"] + st["x_off"]
+            origin = (img - img0) * (st["slot_bytes"] // 4) + iy * w + ix
+            for cl in range(cc):
+                for t in range(9):
+                    inside = (iy + t // 3 >= 0) & (iy + t // 3 < h) & (ix + t % 3 >= 0) & (ix + t % 3 < w)
+                    at = origin + cl * h * w + (t // 3) * w + t % 3
+                    got = np.where(inside, slot[np.clip(at, 0, len(slot) - 1)], np.float32(0))
+                    assert (at[inside] >= 0).all() and (at[inside] < len(slot)).all() and at.min() >= -2 * w - 2 and at.max() < len(slot) + 2 * w + 2
+                    assert np.array_equal(got, padded[img, cl, oy * stride + t // 3, ox * stride + t % 3])
+
+
+def test_what_cannot_be_staged_as_whole_planes():
+    for shape in ((4, 40, 7, 7, 64, 3, 3, 1, 1), (4, 64, 7, 7, 64, 1, 1, 1, 0), (4, 64, 7, 7, 64, 3, 3, 1, 3), (4, 32, 3, 65, 64, 3, 3, 1, 1), (1, 32, 33, 32, 64, 3, 3, 1, 1)):
+        assert staging(shape, 0)["slots"] == 0, shape
+    # pixels of the batch are counted in 32 bits
+    assert staging((1 << 24, 32, 9, 9, 64, 3, 3, 1, 2), 0)["slots"] > 0
+    assert staging((1 << 25, 32, 9, 9, 64, 3, 3, 1, 2), 0)["slots"] == 0

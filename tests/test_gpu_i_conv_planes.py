@@ -173,3 +173,28 @@ def test_planes_beside_an_operator_of_another_cluster_width(rt):
     with pytest.raises(bf.BfuseError) as err:
         pair.fusion(bf.ZIGZAG, 1, 1)
     assert err.value.code == 7
+
+
+@pytest.mark.parametrize("n,ci,hw,co,stride,share", [(8, 256, 14, 130, 1, 2), (32, 128, 7, 64, 1, 2), (40, 64, 15, 96, 2, 2), (24, 128, 7, 256, 2, 3)])
+def test_the_runtime_s_own_choice_against_the_oracle_and_in_a_group(rt, n, ci, hw, co, stride, share):
+    """Shape fields left to the runtime: alone against the oracle, and beside a gathered conv and a GEMM in one launch, bit for bit."""
+    rng = np.random.default_rng(ci + hw + n)
+    planes = wl.conv2d("planes", rng, bf.OP_CONV2D_TF32, n, ci, hw, hw, co, 3, stride, 1)
+    planes.flags = bf.flag_share(share)
+    split = rt.describe("c", planes.op, planes.shape, flags=planes.flags).shape
+    assert split[11] == 3
+    beside = wl.conv2d("gathered", rng, bf.OP_CONV2D_TF32, 2, 32, 9, 9, 40, 3, 1, 1, bn=32, split=split[10], mode=2) if split[10] == 1 else \
+        wl.conv2d("gathered", rng, bf.OP_CONV2D_TF32, 1, 256, 9, 9, 40, 3, 1, 1, bn=32, split=split[10], mode=2)
+    gemm = wl.gemm("g", rng, bf.OP_GEMM_TF32, 1, 70, 64, 64, w_std=1.0, bn=64, split=1)
+    pair = run_and_check(rt, wl.PairSpec("own", planes, beside, "tf32", "hbm"), [(bf.ZIGZAG, 1, 1)])
+    other = wl.DevicePair(rt, wl.PairSpec("own", gemm, beside, "tf32", "hbm"))
+    rt.launch_kernel(other.kernels[0])
+    want = [pair.read_outputs(), other.read_outputs()]
+    for p in (pair, other):
+        p.clear_outputs()
+    group = rt.register_group([pair.kernels[0], other.kernels[0], pair.kernels[1]], bf.ZIGZAG, 1, 1)
+    rt.launch_group(group)
+    got = [pair.read_outputs(), other.read_outputs()]
+    assert rt.read_status() == 0
+    assert np.array_equal(got[0][0][0], want[0][0][0]) and np.array_equal(got[0][1][0], want[0][1][0])
+    assert np.array_equal(got[1][0][0], want[1][0][0])

@@ -77,3 +77,28 @@ def test_slots_describe_the_launch(rt, pattern, split):
             slots = where[lo:lo + per]      # an operator's blocks are handed out in ascending order
             assert (np.diff(slots) == 1).all() and (vb[slots] == np.arange(lo, lo + len(slots))).all()
             assert len(set(sm[slots].tolist())) == 1 and (marks[slots] == marks[slots[0]]).all()
+
+
+@pytest.mark.parametrize("cols", [128, 1024])
+def test_rows_of_infinities_and_nan_beside_finite_ones(rt, cols):
+    """Softmax rows taken two at a time: a row without a finite value, with an infinity or a NaN, or masked but for one value
+    writes what it writes alone, and the rows that share its thread or its warp are not touched."""
+    rng = np.random.default_rng(14)
+    rows = wl.softmax("sm", rng, 6145, cols, 0.125)
+    x = rows.host[0]
+    x[0] = -np.inf
+    x[5, 3] = np.nan
+    x[9, :-1] = -np.inf
+    x[64, 7] = np.inf
+    x[65] = np.finfo(np.float32).min
+    x[6144] = np.nan
+    odd = [0, 5, 64, 6144]
+    g = wl.gemm("g", rng, bf.OP_GEMM_TF32, 2, 200, 256, 64, causal=True, w_std=1.0, bn=256, split=1)
+    pair = run_and_check(rt, wl.PairSpec("odd", rows, g, "tf32", "hbm"), [(bf.ZIGZAG, 1, 1)], check_oracle=False)
+    info = rt.fusion_info(pair.fusion(bf.ZIGZAG, 1, 1))
+    assert info["blocks_per_cta"][0] >= 2
+    y = pair.read_outputs()[0][0]
+    ok = np.ones(len(y), bool)
+    ok[odd] = False
+    assert not np.isfinite(y[odd]).all(1).any()
+    assert np.abs(y[ok].sum(1) - 1).max() <= 1e-5 and y[9, -1] == 1 and np.allclose(y[65], 1 / cols, rtol=1e-5)

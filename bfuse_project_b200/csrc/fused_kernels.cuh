@@ -120,9 +120,9 @@ constexpr int pair_wide_blocks() {
 }
 
 // One CTA, one dispatch slot.  The persistent form is a kernel of its own (fused_queue_kernel): with both in one loop
-// the state that loop carries made every pair with a memory-bound body spill (softmax || LayerNorm 324 bytes a thread in
-// the 40-register build and 44 in the 64-register one, 4 and none without it: 12 launches at 512 tokens 79.3 -> 67.7 us,
-// one at 6007 tokens 64.0 -> 51.4).
+// the state that loop carries made most builds with a memory-bound body spill (61 of 112; softmax || LayerNorm 316 bytes a
+// thread in the 40-register build and 36 in the 64-register one, 4 and none without it: 12 launches at 512 tokens
+// 79.3 -> 67.7 us, one at 6007 tokens 64.0 -> 51.4).
 template <class A, class B, int MINB = pair_min_blocks<A, B>()>
 __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
     fused_block_kernel(const __grid_constant__ DispatchTable t, const __grid_constant__ typename A::Params pa,
@@ -158,7 +158,8 @@ __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
 }
 
 // Persistent CTAs that draw tickets from an atomic counter until the queue is empty.  The last CTA to drain
-// resets the counters, so the next launch on the stream starts from zero without a memset.
+// resets the counters, so the next launch on the stream starts from zero without a memset.  The loop's state spills here as
+// it did in the one kernel (softmax || LayerNorm 280 bytes a thread in 40 registers).
 template <class A, class B>
 __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), (pair_min_blocks<A, B>()))
     fused_queue_kernel(const __grid_constant__ DispatchTable t, const __grid_constant__ typename A::Params pa,

@@ -183,8 +183,6 @@ __host__ __device__ inline bool conv_staged_ring(int smem, int K, int kslot, int
 __host__ __device__ inline int conv_staged_smem_bytes(int header, int slots, int slot_pitch, int wstages) {
   return header + conv_raw_bytes(slots, slot_pitch) + wstages * kUmmaABytes;
 }
-// The whole-plane form with the K range split over a cluster: once the MMAs are done the two rings receive the
-// partial sums of the 16-channel groups a CTA owns, 8 / split groups from each of split CTAs.
 // Raw slots of the whole-plane form in a window of `smem` bytes: what the header and the four weight stages
 // leave, up to 6, never more than a tile loads; 0: the window is too small.
 __host__ __device__ inline int conv_plane_slots(int smem, int Kslice, int cc, int slot_pitch) {
@@ -193,6 +191,8 @@ __host__ __device__ inline int conv_plane_slots(int smem, int Kslice, int cc, in
   while (s > 0 && conv_raw_bytes(s, slot_pitch) > room) --s;
   return s >= (loads < 2 ? loads : 2) ? s : 0;
 }
+// The whole-plane form with the K range split over a cluster: once the MMAs are done the two rings receive the
+// partial sums of the 16-channel groups a CTA owns, 8 / split groups from each of split CTAs.
 constexpr int kConvGroupBytes = 16 * kUmmaBM * 4;   // one CTA's fp32 partial of 16 channels x 128 pixels
 __host__ __device__ constexpr int conv_plane_recv_bytes(int split) { return split > 1 ? 8 * kConvGroupBytes : 0; }
 

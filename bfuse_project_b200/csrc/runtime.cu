@@ -269,7 +269,7 @@ int default_launch(const bfuse_context *ctx, bfuse_kernel_desc *d, std::string *
       if (s[11] == 3 || (s[11] == 0 && s[9] <= 0 && s[10] <= 0 && (long long)s[0] * oh * ow >= kConvBN &&
                          !conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, kConvBN, &rows))) {
         const int imgs = conv_plane_staging(s[0], s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, &planes);
-        if (!imgs && s[11] == 3) { *err = "conv2d: shape[11] = 3 (whole planes) needs a 3 x 3 window, ci a multiple of 32 and four planes of a tile's images in 16 KB"; return BFUSE_ERR_SHAPE; }
+        if (!imgs && s[11] == 3) { *err = "conv2d: shape[11] = 3 (whole planes) needs a 3 x 3 window padded by at most 2, ci a multiple of 32, images at most 64 wide and four planes of a tile's images in 16 KB"; return BFUSE_ERR_SHAPE; }
         const int px_tiles = imgs ? ceil_div(s[0] * oh * ow, planes.tile_px) : 0, co_tiles = ceil_div(s[4], kUmmaBM), tiles = px_tiles * co_tiles;
         int split = s[10];
         if (split <= 0) split = plane_split(tiles, s[1], share, sm);
@@ -542,7 +542,7 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
       ConvStaging planes;
       const int plane_imgs = s[11] == 3 ? conv_plane_staging(s[0], s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, &planes) : 0;
       if (s[11] == 3 && (!plane_imgs || bn != kConvBN || !plane_split_ok(s[10] > 0 ? s[10] : 1, s[1])))
-        return shape_err("shape[11] = 3 (whole planes) needs a 3 x 3 window, ci a multiple of 32, four planes of a tile's images in 16 KB, 128-pixel tiles and 1, 2, 4 or 8 k-slices of whole groups of 32 channels");
+        return shape_err("shape[11] = 3 (whole planes) needs a 3 x 3 window padded by at most 2, ci a multiple of 32, images at most 64 wide, four planes of a tile's images in 16 KB, shape[9] = 128 and 1, 2, 4 or 8 k-slices of whole groups of 32 channels");
       const int split = s[10] > 0 ? s[10] : 1, num_kb = ceil_div(K, ConvUmmaTf32::kBK);
       const int q = plane_imgs ? ceil_div(s[1] / 32, split) * 9 : ceil_div(num_kb, split);
       if (split > 8 || (split - 1) * q >= num_kb) return shape_err("shape[10] (k-slices) must be 1..8 with every k-slice non-empty");
@@ -551,7 +551,7 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
       if (plane_imgs) {
         const int px_tiles = ceil_div(s[0] * oh * ow, planes.tile_px), co_tiles = ceil_div(s[4], kUmmaBM);
         if (split > 1 ? (kd.gx != split * px_tiles || kd.gy != co_tiles || kd.gz != 1) : (long long)kd.gx * kd.gy * kd.gz > (long long)px_tiles * co_tiles)
-          return shape_err("GridDim of a conv staged as whole planes must be (k-slices * ceil(n*oh*ow / 128), ceil(co/128), 1), or hold fewer CTAs with one k-slice");
+          return shape_err("GridDim of a conv staged as whole planes must be (k-slices * ceil(n*oh*ow / pixels per tile), ceil(co/128), 1) -- 128 pixels, or whole images where 128 would need too many planes --, or hold fewer CTAs with one k-slice");
       } else if (s[11] == 1) {
         if ((long long)kd.gx * kd.gy * kd.gz > (long long)ceil_div(oh * ow, tile_px) * ceil_div(s[4], kUmmaBM) * s[0])
           return shape_err("GridDim of a staged conv must not hold more CTAs than the conv has tiles (a CTA takes every grid-size-th tile)");
@@ -561,10 +561,8 @@ int build_params(bfuse_context *ctx, KernelRec &k) {
       k.cluster = split;
       ConvUmmaParams p;
       std::memset(&p, 0, sizeof(p));
-      // Staged (input rows by TMA into a raw ring, repacked in shared memory) when the geometry allows
-      // it and the registered window has room for the raw ring beside the smallest operand ring;
-      // else gathered from global memory.  The raw ring is 3 slots deep, 4 when room is left for a
-      // whole-SM operand ring as well.
+      // The operand mode is what the descriptor says (0: gathered); the registered window has to hold that form's
+      // smallest rings, and what it has beyond them makes them deeper.
       const int min_stages = ceil_div(umma_epilogue_bytes(bn, split, 4), conv_stage_bytes(bn));
       if (s[11] < 0 || s[11] > 3) return shape_err("shape[11] (operand mode) must be 0 (the runtime's choice), 1 (staged), 2 (gathered) or 3 (whole planes)");
       if (s[11] == 1 && (split != 1 || !conv_staging(s[1], s[2], s[3], s[5], s[6], s[7], s[8], oh, ow, bn, &p.st)))

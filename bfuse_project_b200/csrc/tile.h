@@ -27,8 +27,8 @@ struct TileCtx {
   int persistent;       // 1: more tensor-memory allocations may follow in this CTA (work queue: the next
                         // tile; thread split: the other operator), so the allocation permit must be kept
   unsigned tmem_base;   // tmem_given: the tensor-memory columns the CTA already holds for this operator (a persistent
-  int waited = 0;       // 1: an earlier tile of this CTA has waited for the previous kernel
   int tmem_given;       // CTA of the work queue allocates once for all its tickets); the body neither allocates nor frees
+  int waited = 0;       // 1: an earlier tile of this CTA has waited for the previous kernel
 
   // Programmatic dependent launch: the CTA may have started while the previous kernel on the stream
   // was still running.  Every thread calls this before its first access to global memory; what comes
@@ -42,10 +42,12 @@ struct TileCtx {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
 
-  // Is this CTA among those that mostly start under the previous kernel's tail?  Three a SM, of a grid that is not
-  // many rounds long (softmax || LayerNorm of 512 tokens, 12 launches in a row: two a SM 81.3 us, three 79.3, four 80.0,
-  // all 84.0, none 92.8: a CTA that finds the wait over pays for its prefetches and gains nothing).
-  __device__ __forceinline__ bool may_start_early() const { return !waited && !persistent && blockIdx.x < 148 * 3 && gridDim.x <= 148 * 12; }
+  // Is this CTA among those that mostly start under the previous kernel's tail?  Three a SM (of a B200's 148: a hint, any
+  // count is correct), of a grid that is not many rounds long (softmax || LayerNorm of 512 tokens, 12 launches in a row: two
+  // a SM 81.3 us, three 79.3, four 80.0, all 84.0, none 92.8: a CTA that finds the wait over pays for its prefetches
+  // and gains nothing).
+  static constexpr unsigned kSms = 148;
+  __device__ __forceinline__ bool may_start_early() const { return !waited && !persistent && blockIdx.x < kSms * 3 && gridDim.x <= kSms * 12; }
 
   __device__ __forceinline__ void sync() const {
     asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(bar_count) : "memory");

@@ -53,8 +53,9 @@ enum {
                               /* rows by TMA into shared memory, im2col rows written from there into tensor  */
                               /* memory; needs 128-pixel tiles, one k-slice, ci*kh*kw a multiple of 32 and   */
                               /* image rows of 16-byte multiples), 2 gathered from global memory, 3 staged as  */
-                              /* whole image planes (3 x 3 windows, ci a multiple of 32, tiles of 128 pixels of */
-                              /* the whole batch, 1, 2, 4 or 8 k-slices); 0: chosen by bfuse_default_launch  */
+                              /* whole image planes (3 x 3 windows padded by at most 2, ci a multiple of 32,  */
+                              /* images at most 64 wide, tiles of 128 pixels of the whole batch or of whole  */
+                              /* images, 1, 2, 4 or 8 k-slices); 0: chosen by bfuse_default_launch  */
                               /* (staged wherever it can be), which writes 1, 2 or 3 back; a kernel          */
                               /* registered with 0 is gathered, and so is one whose 3 was written back and   */
                               /* that comes with the gathered form's GridDim or a window only that form fits */

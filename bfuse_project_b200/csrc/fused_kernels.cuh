@@ -108,6 +108,10 @@ constexpr int pair_min_blocks() {
                                               : cmin(4, cmax(A::kMinBlocks, B::kMinBlocks));
 }
 
+// Pairs of such bodies test the thread index before both bodies (see fused_block_kernel).
+template <class Op>
+constexpr bool kGuardFirst = false;
+
 // A second, register-richer build of pairs with a memory-bound body, launched when its occupancy
 // still holds the whole fused grid (so nothing is lost in waves).  Two memory-bound bodies: 4 CTAs
 // per SM (64 registers), which let a thread keep more loads in flight than the 40 of the 6-CTA build.
@@ -148,8 +152,14 @@ __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), MINB)
     t.cta_times[3 * (size_t)blockIdx.x] = t_entry;
     t.cta_times[3 * (size_t)blockIdx.x + 1] = global_timer_ns();
   }
-  // guard of the reference: KernelID_ == k && threadIdx.x < B_k (Algorithms.cc:699-717)
-  if (k == 0) {
+  // guard of the reference: KernelID_ == k && threadIdx.x < B_k (Algorithms.cc:699-717).  Two GEMMs: threads past the
+  // operator's block leave here (eight k || v pairs of 333 rows 119.8 -> 118.4 us, twelve Q || K pairs 102.3 -> 101.0
+  // against the test at each body); beside a conv or a CUDA-core body that is 1-5 % slower.
+  if constexpr (kGuardFirst<A> && kGuardFirst<B>) {
+    if (tid >= t.n_thr[k]) return;
+    if (k == 0) run_tile<A>(pa, t, 0, vb, tid, 1, smem);
+    else run_tile<B>(pb, t, 1, vb, tid, 2, smem);
+  } else if (k == 0) {
     if (tid < t.n_thr[0]) run_blocks<A, A::kMemoryBound && B::kUsesTmem && MINB == 2>(pa, t, 0, vb, tid, 1, smem);
   } else {
     if (tid < t.n_thr[1]) run_blocks<B, B::kMemoryBound && A::kUsesTmem && MINB == 2>(pb, t, 1, vb, tid, 2, smem);

@@ -27,6 +27,8 @@ template <> struct OpAt<6> { using type = GemmUmma<0>; };
 template <> struct OpAt<7> { using type = GemmUmma<1>; };
 template <> struct OpAt<8> { using type = ConvAnyTf32; };
 
+template <int KIND> inline constexpr bool kGuardFirst<GemmUmma<KIND>> = true;
+
 struct PairEntry {
   PairLaunchFn block, thread, queue;
   AttrFn block_attr, thread_attr, queue_attr;

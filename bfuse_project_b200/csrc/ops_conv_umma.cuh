@@ -868,10 +868,11 @@ struct ConvUmmaTf32 {
   }
 
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
-    if (p.st.slots > 0) {
-      run_staged<false>(p, c);
-      return;
-    }
+    if (p.st.slots > 0) run_staged<false>(p, c);
+    else run_gathered(p, c);
+  }
+
+  __device__ __forceinline__ static void run_gathered(const Params &p, const TileCtx &c) {
     const int warp = c.tid >> 5, lane = c.tid & 31;
     const int quad = (threadIdx.x >> 5) & 3;
     const int BN = p.bn, kStageBytes = conv_stage_bytes(BN);
@@ -1053,8 +1054,13 @@ struct ConvAnyTf32 : ConvUmmaTf32 {
   // Not inlined: a third form inside run() cost the other two 1 % (batch-256 ResNet branch pair 149.9 -> 151.7 us).
   __device__ __noinline__ static void run_planes(const Params &p, const TileCtx c) { run_staged<true>(p, c); }
   __device__ __forceinline__ static void run(const Params &p, const TileCtx &c) {
-    if (p.plane_imgs > 0) run_planes(p, c);
-    else ConvUmmaTf32::run(p, c);
+    // (in this order: asking for planes first cost LayerNorm || 512 -> 512 on 7 x 7, 32 images, 4 %)
+    if (p.st.slots > 0) {
+      if (p.plane_imgs > 0) run_planes(p, c);
+      else run_staged<false>(p, c);
+    } else {
+      run_gathered(p, c);
+    }
   }
 };
 

@@ -199,11 +199,12 @@ __global__ void __launch_bounds__(cmax(A::kMaxThreads, B::kMaxThreads), (pair_mi
     queue_tmem = *reinterpret_cast<volatile unsigned *>(&queue_tmem_s);
   }
   grid_dependency_wait();   // the ticket counter is global memory
-  // From here on the next kernel may start its CTAs.  Those of a tensor-memory kernel then hold their columns on this SM,
-  // which this CTA's, allocated above, do not wait for.  Keeping them out until the end of the launch costs more (launches in
-  // a row: Q || K 10.8 -> 11.4 us, two 1 x 1 convs of 8 images 11.1 -> 11.9, softmax || GEMM 18.9 -> 19.8) than it
-  // gives to the long ones that gain (softmax || 512 -> 512 on 7 x 7, 32 images, 108 -> 95).
-  grid_launch_dependents();
+  // The next kernel may start its CTAs: from here beside two memory-bound bodies, else from a CTA's first ticket on, where the
+  // body lets it in (from here is 1-2 % slower there).  Those of a tensor-memory kernel then hold their columns on this
+  // SM; this CTA's, allocated above, do not wait for them.  Keeping them out until the end of the launch costs more
+  // (launches in a row: Q || K 10.8 -> 11.4 us, two 1 x 1 convs of 8 images 11.1 -> 11.9, softmax || GEMM 18.9 -> 19.8)
+  // than it gives to the long ones that gain (softmax || 512 -> 512 on 7 x 7, 32 images, 108 -> 95).
+  if constexpr (!A::kUsesTmem && !B::kUsesTmem) grid_launch_dependents();
   __shared__ int ticket_s;
   for (;;) {
     if (tid == 0) ticket_s = (int)atomicAdd(t.queue_ctr, 1u);

@@ -1200,8 +1200,10 @@ int bfuse_register_fusion(bfuse_context *ctx, int kernel1, int kernel2, int patt
   // shared-memory window, mostly half an SM's, and the SM starts the CTAs of such a kernel one after the other.  Where
   // at most two fit an SM anyway the pair takes its register-rich build (the other one spills, and its promise of four
   // CTAs buys nothing), and past two rounds of what is resident the small CTAs take runs of consecutive blocks, two at
-  // a time, so many that both operators together make about two rounds (in one round the partner's slots would idle
-  // once it is done).  Causal QK^T of 6 heads of 1024 tokens beside the softmax of 6 heads (9.6 and 9.1 us alone): 39.0 us,
+  // a time, at least two and as many whole pairs as bring both operators towards two rounds (in one round the partner's
+  // slots would idle once it is done).  Two even where one block a CTA would fit the rounds: 200 LayerNorm blocks beside 1024
+  // GEMM CTAs 26.1 us against 29.3.  Whole pairs rounded down: up to three or four instead of two is between 12 % faster and
+  // 14 % slower by pattern (softmax of 1500 blocks beside 48 CTAs: zig-zag 13.9 -> 15.8 us, range split 17.5 -> 16.6).  Causal QK^T of 6 heads of 1024 tokens beside the softmax of 6 heads (9.6 and 9.1 us alone): 39.0 us,
   // 27.3 with the register-rich build, 21.2 with runs of 4; PV beside the softmax 31.6, 22.8, 18.2 (runs of 2; 20.0 with 4).
   // Smaller windows for the GEMM do not help: with four CTAs an SM in 64 registers QK^T || softmax takes 23-28 us.
   auto memory_bound = [](const KernelRec &k) { return k.desc.op <= BFUSE_OP_ROPE_BF16; };
